@@ -8,6 +8,7 @@
 // kmm_upload_state / kmm_download_state   the Y-pencil U / RK_STORE arrays
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -35,7 +36,8 @@ OpsOffsets ops_offsets(int bw, int ny) {
   o.wlo = o.dyr + ny;
   o.whi = o.wlo + ny;
   o.t0 = o.whi + ny;
-  o.total = o.t0 + (int64_t)ny * (3 * (4 * bw + 1) + (2 * bw + 1) + 2 * bw);
+  o.tt = (o.t0 + (int64_t)ny * (3 * (4 * bw + 1) + (2 * bw + 1) + 2 * bw) + 1) & ~(int64_t)1;
+  o.total = o.tt + (int64_t)ny * op_row_stride(bw);
   return o;
 }
 
@@ -154,6 +156,13 @@ int upload_ops(Handle &h) {
     t += h.ops.l0.size();
     std::memcpy(t, h.ops.u0.data(), h.ops.u0.size() * sizeof(double));
   }
+  for (int r = 0; r < h.ny; ++r) {
+    const int first = std::min(std::max(r - h.bw, 0), h.ny - 1 - 2 * h.bw);
+    for (int j = 0; j <= 2 * h.bw; ++j)
+      for (int d = 0; d < 3; ++d)
+        buf[off.tt + (int64_t)r * op_row_stride(h.bw) + 3 * j + d] =
+            h.ops.off[d][(size_t)r * (4 * h.bw + 1) + 2 * h.bw + first + j - r];
+  }
   KMM_CUDA(cudaMemcpy(h.dops, buf.data(), buf.size() * sizeof(double), cudaMemcpyHostToDevice));
   return KMM_OK;
 }
@@ -217,14 +226,27 @@ int enqueue_substep(Handle &h, int s, cudaStream_t st, cudaEvent_t *ev = nullptr
   };
   int rc;
   if ((rc = rec(KMM_K_BEGIN, [&] { return launch_begin_substep(h, s, st); }))) return rc;
+  // The line solver's factors need this substep's dt alone (and the last substep's solves to be done with
+  // the ones they replace): beside the transforms and hvhg, except in the kernel-by-kernel profile.
+  const bool fork = h.lines && !ev;
+  auto fork_factors = [&]() -> int {
+    KMM_CUDA(cudaEventRecord(h.ev_ffork, st));
+    KMM_CUDA(cudaStreamWaitEvent(h.fside, h.ev_ffork, 0));
+    KMM_CUDA(launch_line_factor(h, s, nullptr, h.fside));
+    KMM_CUDA(cudaEventRecord(h.ev_fjoin, h.fside));
+    return KMM_OK;
+  };
+  if (fork && s != 1 && (rc = fork_factors())) return rc;
   if ((rc = rec(KMM_K_ZINV, [&] { return launch_zinv(h, h.S, h.MID, 3 + h.nsc, st); }))) return rc;
   if ((rc = rec(KMM_K_XPHYS, [&] { return launch_xphys(h, h.MID, s, st); }))) return rc;
   if (s == 1)
     if ((rc = rec(KMM_K_DT, [&] { return launch_update_dt(h, s, st); }))) return rc;
+  if (fork && s == 1 && (rc = fork_factors())) return rc;
   if ((rc = rec(KMM_K_ZFWD, [&] { return launch_zfwd(h, h.MID, h.P, 5 + 3 * h.nsc, h.rescale, !h.mixed, st); })))
     return rc;
   if ((rc = rec(KMM_K_HVHG, [&] { return launch_ws_hvhg(h, s, nullptr, st); }))) return rc;
-  if ((rc = rec(KMM_K_HELMHOLTZ, [&] { return launch_ws_helmholtz(h, s, nullptr, st); }))) return rc;
+  if (fork) KMM_CUDA(cudaStreamWaitEvent(st, h.ev_fjoin, 0));
+  if ((rc = rec(KMM_K_HELMHOLTZ, [&] { return launch_ws_helmholtz(h, s, nullptr, st, fork); }))) return rc;
   if ((rc = rec(KMM_K_ASSEMBLE, [&] { return launch_ws_assemble_only(h, s, nullptr, st); }))) return rc;
   // the mean lines (side stream) join here, outside the assembly's event pair
   KMM_CUDA(launch_ws_join(h, st));
@@ -507,6 +529,9 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&h->fside, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_ffork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_fjoin, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&h->copy, cudaStreamNonBlocking) != cudaSuccess) {
     set_error("cudaStreamCreate failed");
@@ -529,15 +554,25 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   if ((rc = dalloc(*h, &h->vwall, 2 * (size_t)h->nmodes))) return fail(rc);
   if ((rc = dalloc(*h, &h->zc, (8 + 2 * x2) * (size_t)h->ns))) return fail(rc);
   if ((rc = dalloc(*h, &h->ec, (9 + 2 * x2) * (size_t)h->ns))) return fail(rc);
-  if ((rc = dalloc(*h, &h->xr, 6 * (size_t)h->ns))) return fail(rc);
-  if ((rc = dalloc(*h, &h->ub, (3 + x2) * (size_t)split_ub_role(*h)))) return fail(rc);
-  if ((rc = dalloc(*h, &h->vf, (size_t)vop_factor_doubles(*h)))) return fail(rc);
+  h->lines = line_solver_fits(*h);
+  // (the pressure solve keeps its U factors in the first role's region of ub)
+  if ((rc = dalloc(*h, &h->ub, (h->lines ? 1 : 3 + x2) * (size_t)split_ub_role(*h)))) return fail(rc);
   if ((rc = dalloc(*h, &h->dvw, 3 * (size_t)h->nmodes))) return fail(rc);
+  if (h->lines) {
+    const size_t sets = (size_t)(1 + h->nsc) * (factor_cache_possible(*h) ? 3 : 1);
+    if ((rc = dalloc(*h, &h->lf, sets * (size_t)tile_factor_doubles(*h)))) return fail(rc);
+    if ((rc = dalloc(*h, &h->lvf, (size_t)tile_factor_doubles(*h)))) return fail(rc);
+  } else {
+    if ((rc = dalloc(*h, &h->xr, 6 * (size_t)h->ns))) return fail(rc);
+    if ((rc = dalloc(*h, &h->vf, (size_t)vop_factor_doubles(*h)))) return fail(rc);
+  }
   if (factor_cache_possible(*h)) {
-    // per substep: the two Helmholtz operators' factors, the four influence lines, v_h's walls
-    if ((rc = dalloc(*h, &h->hf, 6 * (size_t)vop_factor_doubles(*h)))) return fail(rc);
-    if ((rc = dalloc(*h, &h->hinf, 12 * (size_t)h->ns))) return fail(rc);
-    if ((rc = dalloc(*h, &h->hdvh, 3 * (size_t)h->nmodes))) return fail(rc);
+    if (!h->lines) {
+      // per substep: the two Helmholtz operators' factors, the four influence lines, v_h's walls
+      if ((rc = dalloc(*h, &h->hf, 6 * (size_t)vop_factor_doubles(*h)))) return fail(rc);
+      if ((rc = dalloc(*h, &h->hinf, 12 * (size_t)h->ns))) return fail(rc);
+      if ((rc = dalloc(*h, &h->hdvh, 3 * (size_t)h->nmodes))) return fail(rc);
+    }
     if ((rc = dalloc(*h, &h->fcdt, 3))) return fail(rc);
     const double none[3] = {NAN, NAN, NAN};  // no dt cached yet
     if (cudaMemcpy(h->fcdt, none, sizeof(none), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -545,7 +580,7 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
       return fail(KMM_ERR_CUDA);
     }
   }
-  if ((rc = dalloc(*h, &h->w00, (3 + x2) * (size_t)h->ny * (8 + 2 * h->bw)))) return fail(rc);
+  if ((rc = dalloc(*h, &h->w00, (size_t)mean_doubles(*h)))) return fail(rc);
   if ((rc = dalloc(*h, &h->staging, 10 * h->ns))) return fail(rc);
   if ((rc = dalloc(*h, &h->dsc, 1))) return fail(rc);
   if (cudaMemset(h->S, 0, sizeof(double2) * nfld * h->ns) != cudaSuccess ||
@@ -576,7 +611,7 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
     return fail(KMM_ERR_CUDA);
   }
   {
-    // the v operator depends on k^2 alone: factor it once for the run
+    // shared-memory limits; and the v operator depends on k^2 alone: factor it once for the run
     cudaError_t e = launch_vop_factor(*h, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) {
@@ -590,7 +625,7 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   // (384x257x384: x pass 8.54 -> 6.15 ms, 17.0 -> 19.4 steps/s, the tuner's pick there)
   if (!h->mixed && h->nsc == 2 && h->nx32 >= 576) h->tune.x = 1;
   // with a fixed time step the Helmholtz sweeps read their operators' cached factors
-  h->tune.fcache = h->hf ? 1 : 0;
+  h->tune.fcache = h->fcdt ? 1 : 0;
   // the z transforms stage their input tiles through TMA where the grid allows the tile map
   // (0.062 -> 0.054 ms y_to_x, 312 -> 315 steps/s at 192x129x192 mixed, same-box A/B)
   h->tune.ztma = z_tma_possible(*h, h->tune.z) ? 1 : 0;
@@ -607,15 +642,19 @@ int kmm_destroy(kmm_handle *hh) {
   if (h->graph) cudaGraphDestroy(h->graph);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->side) cudaStreamSynchronize(h->side);
+  if (h->fside) cudaStreamSynchronize(h->fside);
   adjoint_free(*h);
   void *ptrs[] = {h->S, h->RK, h->P, h->MID, h->dops, h->gains, h->vwall, h->zc,
                   h->ec, h->xr, h->ub, h->vf, h->dvw, h->w00, h->staging, h->stat,
-                  h->mid64, h->p64, h->hf, h->hinf, h->hdvh, h->fcdt, h->fftpos, h->tw64, h->tw32, h->dsc};
+                  h->mid64, h->p64, h->hf, h->hinf, h->hdvh, h->fcdt, h->lf, h->lvf, h->fftpos, h->tw64, h->tw32, h->dsc};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h->copy) cudaStreamSynchronize(h->copy);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   if (h->ev_join) cudaEventDestroy(h->ev_join);
+  if (h->ev_ffork) cudaEventDestroy(h->ev_ffork);
+  if (h->ev_fjoin) cudaEventDestroy(h->ev_fjoin);
+  if (h->fside) cudaStreamDestroy(h->fside);
   for (auto ev : h->ev_io)
     if (ev) cudaEventDestroy(ev);
   if (h->copy) cudaStreamDestroy(h->copy);

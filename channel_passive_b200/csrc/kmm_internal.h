@@ -27,6 +27,8 @@ constexpr int kMaxPass = 8;
 constexpr int kNumMoments = 18;
 // Spectra per direction of a statistics step (stats.cu k_spectra).
 constexpr int kNumSpec = KMM_STAT_NSPEC;
+// Modes whose lines a block of the line solver holds (lines.cuh).
+constexpr int kTileModes = 8;
 constexpr int kMinBw = 2;
 constexpr int kMaxBw = 7;
 
@@ -137,11 +139,19 @@ struct Handle {
   double *hinf = nullptr;                  // [substep][4][ny][nmodes] influence lines
   double2 *hdvh = nullptr;                 // [substep][nmodes] (dv_h(1), dv_h(n))
   double *fcdt = nullptr;                  // [substep] the dt the cache holds (NaN: none)
+  // The line solver's factors instead of hf, hinf, hdvh, vf (lines.cuh TileFac, tile_factor_doubles each):
+  // of theta's operator, the one g and phi share and a second scalar's, made every substep, or with
+  // the factor cache per substep and dt; and of v's.
+  bool lines = false;                      // the Helmholtz solves run in line_solver.cu (line_solver_fits)
+  double *lf = nullptr, *lvf = nullptr;
+  int smem_optin = 0, smem_sm = 0;         // the device's shared memory: most of a block, of an SM
   double *stat = nullptr;                  // statistics buffers (stat_layout), made on first use
   double2 *mid64 = nullptr, *p64 = nullptr;  // mixed handles: FP64 slab [6][nm] and products [6][ns]
                                              // of the pressure / statistics pass, made on first use
   cudaStream_t side = nullptr;             // mean-mode lines run here, forked from / joined to stream
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t fside = nullptr;            // the line solver's factors, forked from / joined to stream
+  cudaEvent_t ev_ffork = nullptr, ev_fjoin = nullptr;
   cudaStream_t copy = nullptr;             // host <-> device copies of kmm_step_host, beside stream
   cudaEvent_t ev_io[9] = {};               // its per-field hand-offs between copy and stream
   double2 *staging = nullptr;              // [7][nz][nxh][ny] reference-layout staging
@@ -162,9 +172,20 @@ struct Handle {
 struct OpsOffsets {
   int64_t d0, d1, d2, d0lu, integ, dyr, wlo, whi;
   int64_t t0;  // offset tables T0, T1, T2 [ny][4bw+1], then the D0 profile LU L0 [ny][2bw+1], U0 [ny][2bw]
+  int64_t tt;  // rows of D0, D1, D2 over their own columns: [ny][op_row_stride], [2bw+1][3] of it used
   int64_t total;
 };
 OpsOffsets ops_offsets(int bw, int ny);
+// Doubles of a row of OpsOffsets::tt: whole 16-byte units (bulk copies), and such that the same entry
+// of four rows lies in four different shared-memory banks.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int op_row_stride(int bw) {
+  int r = 3 * (2 * bw + 1) + 1;
+  while (2 * r % 16 == 0) r += 2;
+  return r;
+}
 
 // Kernel launchers (transforms.cu, labs_kernels.cu).
 // fp64: compute in FP64 on a mixed handle too (mid then holds double2 lines; zfwd writes double2).
@@ -244,7 +265,9 @@ cudaError_t launch_wavespace_split(Handle &h, int substep, const double *dt_over
 // The three parts of launch_wavespace_split (control probe + mean fork + hvhg; Helmholtz;
 // assembly + mean join), for per-kernel timing.
 cudaError_t launch_ws_hvhg(Handle &h, int substep, const double *dt_override, cudaStream_t st);
-cudaError_t launch_ws_helmholtz(Handle &h, int substep, const double *dt_override, cudaStream_t st);
+// (factored: the line solver's factors of this substep are already on st)
+cudaError_t launch_ws_helmholtz(Handle &h, int substep, const double *dt_override, cudaStream_t st,
+                                bool factored = false);
 cudaError_t launch_ws_assemble(Handle &h, int substep, const double *dt_override, cudaStream_t st);
 // The assembly kernel alone, and the join of the mean lines (the side stream) onto st; the
 // kernel-by-kernel profile records the assembly without the join.
@@ -276,9 +299,22 @@ cudaError_t launch_statistics(Handle &h, cudaStream_t st);
 // whole (L then U), and the kernel that fills it once per handle.
 int64_t vop_lband_doubles(const Handle &h);
 int64_t vop_factor_doubles(const Handle &h);
+// The line solver (line_solver.cu): whether it takes h's grid (called once, by kmm_create, which also
+// learns the device's shared memory from it), doubles of one operator's LU of every mode in its layout,
+// its set-up (shared-memory limits, v's factors), the factors of a substep (they need its dt alone) and
+// the Helmholtz part of a substep.
+bool line_solver_fits(Handle &h);
+int64_t tile_factor_doubles(const Handle &h);
+cudaError_t prepare_line_solver(Handle &h, cudaStream_t st);
+cudaError_t launch_line_factor(Handle &h, int substep, const double *dt_ptr, cudaStream_t st);
+cudaError_t launch_line_solver(Handle &h, int substep, const double *dt_ptr, cudaStream_t st);
 // Whether the handle can cache the Helmholtz factors: a fixed time step and one scalar.
 bool factor_cache_possible(const Handle &h);
 cudaError_t launch_vop_factor(Handle &h, cudaStream_t st);
+// The mean lines (mean.cu): doubles of their work space, their set-up and launch.
+int64_t mean_doubles(const Handle &h);
+cudaError_t prepare_mean(Handle &h);
+cudaError_t launch_mean(Handle &h, int substep, const double *dt_ptr, cudaStream_t st);
 // Doubles of U factor storage per solver role.
 int64_t split_ub_role(const Handle &h);
 // Operator tables in shared memory for the hvhg and Helmholtz kernels (their bytes per block,

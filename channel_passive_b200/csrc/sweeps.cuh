@@ -350,7 +350,8 @@ __device__ __forceinline__ void bwd_emit(int n, UF ufn, Zin zin, Emit emit, Pf p
 // 2BW+1..n-BW only touch U(p, p+e) with e <= BW of the last BW rows, which stay in a register
 // window; the first 2BW and last BW rows read U back from ust.
 // With KEEP_L, step() leaves row r's L (Lk[d] = L(r, r-d), Lk[0] = 1 / L(r, r)) in Lk.
-template <int BW, int NC, int NR, bool KEEP_L = false>
+// US stores U (get / set like UBand).
+template <int BW, int NC, int NR, bool KEEP_L = false, typename US = UBand<BW>>
 struct LuSweep {
   static constexpr int W = 2 * BW;
   static constexpr int NCc = NC > 0 ? NC : 1, NRr = NR > 0 ? NR : 1;
@@ -358,10 +359,10 @@ struct LuSweep {
   double wr[NRr][W];
   double Uw[BW][BW];  // Uw[dp-1][e-1] = U(r-dp, r-dp+e)
   double Lk[KEEP_L ? W + 1 : 1];
-  UBand<BW> ust;
+  US ust;
   int n;
 
-  __device__ __forceinline__ void init(int n_, UBand<BW> u) {
+  __device__ __forceinline__ void init(int n_, US u) {
     n = n_;
     ust = u;
 #pragma unroll

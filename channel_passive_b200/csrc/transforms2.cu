@@ -12,6 +12,7 @@
 #include "fft2.cuh"
 #include "kmm_internal.h"
 #include "stats.cuh"
+#include "tma.cuh"
 
 namespace kmm {
 
@@ -39,37 +40,12 @@ __device__ __forceinline__ int zpad_src(int p, int nh) { return p < nh ? p : (p 
 // A block's input tile (its KB kx columns of all rows of one (field, y) plane) is copied into
 // shared memory as 3-D tensor boxes of (2 KB scalars, tile_rows(n) rows, 1 plane); the copies
 // complete on an mbarrier whose wait has an iteration limit.
-constexpr int kTmaWaitIters = 1 << 20;
-
 // Rows of one TMA box over n rows: n split into ceil(n / 256) equal boxes (0 if they are not equal).
 __host__ __device__ constexpr int tile_rows(int n) {
   const int nb = (n + 255) / 256;
   return n % nb == 0 ? n / nb : 0;
 }
 
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, unsigned phase) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait for phase 0 of `bar`; false if it gave up
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar) {
-  for (int it = 0; it < kTmaWaitIters; ++it)
-    if (mbar_try_wait(bar, 0)) return true;
-  return false;
-}
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"

@@ -401,7 +401,7 @@ int kmm_set_tuning(kmm_handle *hh, const kmm_tuning *t) {
                        (t->helm_stage_ahead == 1 || t->helm_stage_ahead == 2) &&
                        helm_shape_fits(h, hg, t->helm_tables_shared, t->helm_stage_ahead);
   const bool tma_ok = t->z_tma == 0 || (t->z_tma == 1 && zv >= 0 && z_tma_possible(h, zv));
-  const bool fc_ok = t->factor_cache == 0 || (t->factor_cache == 1 && h.hf);
+  const bool fc_ok = t->factor_cache == 0 || (t->factor_cache == 1 && h.fcdt);
   if (zv < 0 || xv < 0 || g == 0 || (g == 2 && h.nsc != 1) || (t->u_layout != 0 && t->u_layout != 1) || !asm_ok ||
       !tab_ok || !helm_ok || !tma_ok || !fc_ok) {
     set_error("kmm_set_tuning: a requested shape is not among this grid's candidates (see kmm_autotune)");

@@ -25,11 +25,11 @@
 //   solve_v_f.f90:142), so role 3 carries one real chain.
 // k_assemble, one thread per (y, mode): C1, C2 from the wall derivatives (solve_v_f.f90:293-298),
 //   v, dv/dy, RK_STORE 2 completion, then u and w (solve_u_w.f90:27-38).
-// k_mean, three threads on a forked stream: wave00.f90:41-714 for U, W and Theta.
+// k_mean (mean.cu) on a forked stream: wave00.f90:41-714 for U, W and Theta.
 #include <cuda_runtime.h>
 
 #include "kmm_internal.h"
-#include "sweeps.cuh"
+#include "lines.cuh"
 
 namespace kmm {
 
@@ -37,22 +37,6 @@ namespace {
 
 constexpr int kLanes = 32;  // modes per block; one warp per role
 constexpr int kRoles = 4;
-
-// Lines k_hvhg hands to k_helmholtz.  The six nonlinear-term lines H_HV0..H_V3 are combinations
-// of the products and are stored at the products' precision PT (float2 in the mixed path, packed
-// at (PT *)hl + i * ns); the substep-1 lines H_DP, H_DT, H_DG (D2 D0^{-1} of the FP64 RK stores)
-// stay double2 at hl + i * ns.
-// A second passive scalar adds H_HT2 (its nonlinear term, at PT like H_HT) and H_DT2 (substep 1,
-// double2 like H_DT).
-enum HLine { H_HV0 = 0, H_HT, H_G2, H_V2, H_G3, H_V3, H_DP, H_DT, H_DG, H_HT2, H_DT2, H_COUNT };
-
-// Low-storage RK3 coefficients alpha, beta, gamma, zeta of substeps 1-3
-// (RK3_initialize, module_runge_kutta.f90:34-45).
-__constant__ double c_rk[4][3] = {{29.0 / 96.0, -3.0 / 40.0, 1.0 / 6.0},
-                                  {37.0 / 160.0, 5.0 / 24.0, 1.0 / 6.0},
-                                  {8.0 / 15.0, 5.0 / 12.0, 3.0 / 4.0},
-                                  {0.0, -17.0 / 60.0, -5.0 / 12.0}};
-__device__ __forceinline__ double rkc(int c, int s) { return c_rk[c - 1][s - 1]; }
 
 struct SplitArgs {
   int ny, nxh, nz, substep;
@@ -113,64 +97,8 @@ __device__ __forceinline__ UBand<BW> role_uband(const SplitArgs &a, int role, in
                         : make_uband<BW>(base, BW * a.nmodes, a.nmodes, BW * a.ns, a.nmodes);
 }
 
-template <typename PT> __device__ __forceinline__ double2 ldp(const PT *p);
-template <> __device__ __forceinline__ double2 ldp<double2>(const double2 *p) { return *p; }
-template <> __device__ __forceinline__ double2 ldp<float2>(const float2 *p) {
-  const float2 v = *p;
-  return make_double2((double)v.x, (double)v.y);
-}
-
-struct ModeK {
-  double kx, kz, k2;
-};
 __device__ __forceinline__ ModeK mode_k(const SplitArgs &a, int64_t m) {
-  const int mi = (int)m, kzi = mi / a.nxh, kxi = mi - kzi * a.nxh;
-  const int kzint = (kzi <= a.nz / 2) ? kzi : kzi - a.nz;  // set_waveno
-  ModeK k;
-  k.kx = kxi * a.lmfxr;                                   // wavespace.f90:69
-  k.kz = kzint * a.lmfzr;
-  k.k2 = k.kx * k.kx + k.kz * k.kz;
-  return k;
-}
-
-// A = ca D0 - cb D2 with the Dirichlet first / last rows, as an offset row (|e| <= BW only
-// for a centre row, which is never a wall row).
-template <int BW>
-__device__ __forceinline__ void helm_row(const Tabs<BW> &tb, int r, int n, double ca, double cb, double *out,
-                                         bool centre) {
-  const double *r0 = trow<BW>(tb.t0, r), *r2 = trow<BW>(tb.t2, r);
-  if (centre) {
-#pragma unroll
-    for (int e = -BW; e <= BW; ++e) out[e + 2 * BW] = ca * r0[e] - cb * r2[e];
-    return;
-  }
-  if (r == 1 || r == n) {
-#pragma unroll
-    for (int e = -2 * BW; e <= 2 * BW; ++e) out[e + 2 * BW] = 0.0;
-    out[2 * BW] = ca * r0[0] - cb * r2[0];
-    return;
-  }
-#pragma unroll
-  for (int e = -2 * BW; e <= 2 * BW; ++e) out[e + 2 * BW] = ca * r0[e] - cb * r2[e];
-}
-
-// (D2 - k^2 D0) with the wall rows replaced by D0 (v given there), solve_v_f.f90:95-140.
-template <int BW>
-__device__ __forceinline__ void vrow(const Tabs<BW> &tb, int r, int n, double k2, double *row, bool centre) {
-  const double *r0 = trow<BW>(tb.t0, r), *r2 = trow<BW>(tb.t2, r);
-  if (centre) {
-#pragma unroll
-    for (int e = -BW; e <= BW; ++e) row[e + 2 * BW] = -k2 * r0[e] + r2[e];
-    return;
-  }
-  if (r == 1 || r == n) {
-#pragma unroll
-    for (int e = -2 * BW; e <= 2 * BW; ++e) row[e + 2 * BW] = 0.0;
-    row[2 * BW] = r0[0];
-    return;
-  }
-#pragma unroll
-  for (int e = -2 * BW; e <= 2 * BW; ++e) row[e + 2 * BW] = -k2 * r0[e] + r2[e];
+  return kmm::mode_k((int)m, a.nxh, a.nz, a.lmfxr, a.lmfzr);
 }
 
 // A staged nonlinear-term unit, widened to double2.
@@ -847,149 +775,6 @@ __global__ void __launch_bounds__(512) k_assemble(SplitArgs a) {
   S[2 * ns + o] = zadd(zmul(kxx, g), zmul(kzz, dv));
 }
 
-// ------------------------------------------------------------------------------------------
-// k_mean: wave00.f90 for one mean line per thread: U (line 0: forced, Galilean shift),
-// W (line 1: phi = 0), Theta (line 2: nu/pr, forced to the bulk value).
-struct MeanArgs {
-  int ny, substep, nsc;
-  int64_t nmodes, ns;
-  double2 *S, *RK;
-  const void *P;
-  double *w00;
-  const double *tabs, *integ;
-  double nu, pr, bulk_u, bulk_w, bulk_t, u_gal;
-  double pr2, bulk_t2;  // a second passive scalar (line 3)
-  DevScalars *dsc;
-  const double *dt_ptr;
-};
-
-template <int BW, typename PT>
-__global__ void k_mean(MeanArgs a) {
-  const int line = threadIdx.x;
-  if (line >= 2 + a.nsc || a.dsc->err) return;
-  const Tabs<BW> tb = tabs_at<BW>(a.tabs, a.ny);
-  const int n = a.ny, s = a.substep;
-  const int64_t ns = a.ns;
-  const double dt = *a.dt_ptr;
-  // line 3: a second passive scalar, the theta block with its own Prandtl number and bulk value
-  const double visc = (line == 2) ? a.nu / a.pr : (line == 3) ? a.nu / a.pr2 : a.nu;
-  const double gal = (line == 0) ? a.u_gal : 0.0;
-  const double bulk = (line == 0) ? a.bulk_u : (line == 1) ? a.bulk_w : (line == 2) ? a.bulk_t : a.bulk_t2;
-  const int pslot = (line == 0) ? 1 : (line == 1) ? 3 : (line == 2) ? 6 : 9;  // uv, vw, v theta, v theta2
-  const PT *P = reinterpret_cast<const PT *>(a.P) + pslot * ns;
-  const DLine store{a.RK + line * ns, a.nmodes};
-  const DLine out{a.S + (line == 0 ? 0 : line == 1 ? 2 : line == 2 ? 3 : 4) * ns, a.nmodes};
-  const int64_t per = 8 * (int64_t)n + 2 * BW * (int64_t)n;  // doubles per line thread
-  double *base = a.w00 + line * per;
-  const DLine Zf{reinterpret_cast<double2 *>(base), 1}, Zs{reinterpret_cast<double2 *>(base) + n, 1};
-  const DLine R{reinterpret_cast<double2 *>(base) + 2 * n, 1}, DF{reinterpret_cast<double2 *>(base) + 3 * n, 1};
-  const UBand<BW> ub = make_uband<BW>(base + 8 * (int64_t)n, 1, n);
-  auto ufix = [&](int r, int e) { return tb.u0[(r - 1) * 2 * BW + e - 1]; };
-  // D0 solves: the flux product (and the store at substep 1)
-  fwd_fixed<BW, 2>(tb, n,
-      [&](int r, double2 *b) {
-        b[0] = ldp<PT>(P + (r - 1) * (int)a.nmodes);
-        b[1] = (s == 1) ? store.ld(r) : z2(0.0, 0.0);
-      },
-      [&](int r, const double2 *z) { Zf.st(r, z[0]); Zs.st(r, z[1]); },
-      [&](int r) {
-        pf_l1(P + (r - 1) * (int)a.nmodes);
-        pf_l1(store.p + (r - 1) * (int)a.nmodes);
-      });
-  auto pfw = [&](const DLine &l, int r) { pf_l1(l.p + (r - 1)); };
-  bwd_emit<BW, 2, 0>(n, ufix,
-      [&](int r, double2 *zc, double *) { zc[0] = Zf.ld(r); zc[1] = Zs.ld(r); },
-      [&](int q, int r, const double2 (&wc)[2][2 * BW + 1], const double (&)[1][2 * BW + 1]) {
-        const double2 d = mvc<BW>(tb.t1, q, r, wc[0]);  // d/dy of the flux
-        DF.st(q, d);
-        double2 b;
-        const double gamma = dt * rkc(3, s);
-        if (s == 1) {
-          const double alpha = dt * rkc(1, s) * visc;
-          b = zsub(zadd(store.ld(q), zscale(alpha, mvc<BW>(tb.t2, q, r, wc[1]))), zscale(gamma, d));
-        } else {
-          b = zsub(store.ld(q), zscale(gamma, d));
-        }
-        // wave00.f90:169-173: zero wall rows, interior real part + u_gal, imaginary part 1
-        R.st(q, (q == 1 || q == n) ? z2(0.0, 0.0) : z2(b.x + gal, 1.0));
-      },
-      [&](int r) {
-        pfw(Zf, r);
-        pfw(Zs, r);
-        if (r <= n - 2 * BW) pf_l1(store.p + (r + BW - 1) * (int)a.nmodes);
-      });
-  // (D0 - beta D2) c = rhs, Dirichlet rows
-  const double beta = dt * rkc(2, s) * visc;
-  lu_fwd<BW, 1, 0>(n, [&](int r, double *row, bool c) { helm_row<BW>(tb, r, n, 1.0, beta, row, c); },
-      [&](int r, double2 *bc, double *) { bc[0] = R.ld(r); },
-      [&](int r, const double2 *zc, const double *) { R.st(r, zc[0]); }, ub, [&](int r) { pfw(R, r); });
-  // backward substitution storing the coefficients; the integral (LABS_integration) runs along,
-  // summed from row n down
-  double2 integral = z2(0.0, 0.0);
-  {
-    double2 w[2 * BW + 1];
-#pragma unroll
-    for (int j = 0; j <= 2 * BW; ++j) w[j] = z2(0.0, 0.0);
-    for (int r = n; r >= 1; --r) {
-      if (r > kPrefetchRows) {
-        pfw(R, r - kPrefetchRows);
-#pragma unroll
-        for (int e = 1; e <= BW; ++e) pf_l1(ub.p + (e - 1) * (int)n + (r - kPrefetchRows - 1));
-      }
-#pragma unroll
-      for (int j = 2 * BW; j >= 1; --j) w[j] = w[j - 1];
-      double2 acc = R.ld(r);
-#pragma unroll
-      for (int e = 1; e <= 2 * BW; ++e) {
-        const double u = ub.get(r, e);
-        acc.x -= u * w[e].x;
-        acc.y -= u * w[e].y;
-      }
-      w[0] = acc;
-      R.st(r, acc);
-      integral = zadd(integral, zscale(__ldg(a.integ + r - 1), acc));
-    }
-  }
-  double phi = (bulk - 0.5 * integral.x) / (0.5 * integral.y);  // calculate_phi
-  if (line == 1) phi = 0.0;                                       // wave00.f90:396
-  // c = Re c + phi Im c (real), formed where it is read: the wall stresses and the last sweep
-  auto creal = [&](int r) {
-    const double2 c = R.ld(r);
-    return c.x + phi * c.y;
-  };
-  if (s == 3) {
-    const double *r1 = trow<BW>(tb.t1, 1), *rn = trow<BW>(tb.t1, n);
-    const double wall = r1[0] * creal(1) + r1[1] * creal(2) - rn[-1] * creal(n - 1) - rn[0] * creal(n);
-    if (line == 0) a.dsc->wall_shear_stress = 0.5 * a.nu * wall;
-    if (line == 2) a.dsc->wall_theta_stress = 0.5 * a.nu / a.pr * wall;
-    if (line == 3) a.dsc->wall_theta_stress2 = 0.5 * a.nu / a.pr2 * wall;
-  }
-  if (line == 0) a.dsc->phi_dpdx[s - 1] = phi;
-  if (line == 2) a.dsc->phi_dtdx[s - 1] = phi;
-  if (line == 3) a.dsc->phi_dtdx2[s - 1] = phi;
-  bwd_emit<BW, 1, 0>(n, [&](int, int) { return 0.0; },
-      [&](int r, double2 *zc, double *) { zc[0] = z2(creal(r), 0.0); },
-      [&](int q, int r, const double2 (&wc)[1][2 * BW + 1], const double (&)[1][2 * BW + 1]) {
-        double2 prof = mvc<BW>(tb.t0, q, r, wc[0]);
-        prof.x -= gal;
-        out.st(q, prof);
-        if (s != 3) {
-          const double alpha = dt * rkc(1, s + 1) * visc, zeta = dt * rkc(4, s + 1);
-          store.st(q, zsub(zadd(zscale(alpha, mvc<BW>(tb.t2, q, r, wc[0])), prof), zscale(zeta, DF.ld(q))));
-        } else {
-          store.st(q, prof);
-        }
-      },
-      [&](int r) {
-        pfw(R, r);
-        if (r <= n - 2 * BW) pfw(DF, r + BW);
-      });
-  if (line == 1) {  // v mean = 0 (wave00.f90:462)
-    const DLine Sv{a.S + ns, a.nmodes};
-    for (int r = 1; r <= n; ++r) Sv.st(r, z2(0.0, 0.0));
-  }
-}
-
 // part 0: fork the mean lines to h.side, then k_hvhg; part 1: k_helmholtz; part 2: k_assemble,
 // then join h.side back to st.
 template <int BW>
@@ -1040,29 +825,6 @@ cudaError_t split_bw(Handle &h, int part, int substep, const double *dt_ptr, cud
   a.xinf = fc ? h.hinf + 4 * (int64_t)(substep - 1) * h.ns : h.xr + h.ns;
   a.dvh = fc ? h.hdvh + (int64_t)(substep - 1) * h.nmodes : h.dvw + 2 * h.nmodes;
 
-  MeanArgs ma;
-  ma.ny = h.ny;
-  ma.substep = substep;
-  ma.nsc = h.nsc;
-  ma.pr2 = h.cfg.pr2;
-  ma.bulk_t2 = h.cfg.bulk_t2;
-  ma.nmodes = h.nmodes;
-  ma.ns = h.ns;
-  ma.S = h.S;
-  ma.RK = h.RK;
-  ma.P = h.P;
-  ma.w00 = h.w00;
-  ma.tabs = a.tabs;
-  ma.integ = h.dops + off.integ;
-  ma.nu = h.cfg.nu;
-  ma.pr = h.cfg.pr;
-  ma.bulk_u = h.cfg.bulk_vel_u;
-  ma.bulk_w = h.cfg.bulk_vel_w;
-  ma.bulk_t = h.cfg.bulk_t;
-  ma.u_gal = h.cfg.u_gal;
-  ma.dsc = h.dsc;
-  ma.dt_ptr = dtp;
-
   cudaError_t e;
   const int G = a.groups;
   const unsigned blocks = (unsigned)((h.nmodes + (int64_t)kLanes * G - 1) / ((int64_t)kLanes * G));
@@ -1071,9 +833,7 @@ cudaError_t split_bw(Handle &h, int part, int substep, const double *dt_ptr, cud
     // the mean lines touch only mode 0, which the split kernels skip: run them beside those
     if ((e = cudaEventRecord(h.ev_fork, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(h.side, h.ev_fork, 0)) != cudaSuccess) return e;
-    if (h.mixed) k_mean<BW, float2><<<1, 32, 0, h.side>>>(ma);
-    else k_mean<BW, double2><<<1, 32, 0, h.side>>>(ma);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_mean(h, substep, dtp, h.side)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(h.ev_join, h.side)) != cudaSuccess) return e;
     if (h.nsc == 2) {
       if (h.mixed) k_hvhg<BW, float2, 2><<<blocks, kLanes * (kRoles + 1), tsm, st>>>(a);
@@ -1300,7 +1060,9 @@ cudaError_t launch_vop_factor(Handle &h, cudaStream_t st) {
   // shared memory: allow every instantiation of this BW the device's opt-in maximum (the
   // attribute only bounds a launch; each launch asks for what it uses)
   cudaError_t e = set_solver_smem_limits(h);
+  if (e == cudaSuccess) e = prepare_mean(h);
   if (e != cudaSuccess) return e;
+  if (h.lines) return prepare_line_solver(h, st);
   switch (h.bw) {
     case 2: k_vop_factor<2><<<blocks, 128, 0, st>>>(a); break;
     case 3: k_vop_factor<3><<<blocks, 128, 0, st>>>(a); break;
@@ -1317,11 +1079,16 @@ cudaError_t launch_ws_hvhg(Handle &h, int substep, const double *dt_ptr, cudaStr
   return split_part(h, 0, substep, dt_ptr, st);
 }
 
-cudaError_t launch_ws_helmholtz(Handle &h, int substep, const double *dt_ptr, cudaStream_t st) {
+cudaError_t launch_ws_helmholtz(Handle &h, int substep, const double *dt_ptr, cudaStream_t st, bool factored) {
+  if (h.lines) {
+    const cudaError_t e = factored ? cudaSuccess : launch_line_factor(h, substep, dt_ptr, st);
+    return e == cudaSuccess ? launch_line_solver(h, substep, dt_ptr, st) : e;
+  }
   return split_part(h, 1, substep, dt_ptr, st);
 }
 
 cudaError_t launch_ws_assemble_only(Handle &h, int substep, const double *dt_ptr, cudaStream_t st) {
+  if (h.lines) return cudaSuccess;  // part of its kernel
   return split_part(h, 2, substep, dt_ptr, st);
 }
 

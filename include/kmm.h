@@ -94,6 +94,8 @@ typedef struct kmm_info {
 
 /* Launch shapes chosen by kmm_autotune (the hand-tuned defaults before it runs), and the
  * measured device time (ms) of every candidate it tried. */
+/* On grids of up to 12000 modes the Helmholtz solves run in the line solver, which has one shape:
+ * u_layout, assemble_threads and the helm_* fields are checked and reported there and change nothing. */
 typedef struct kmm_tuning {
   int32_t z_lines_per_block;  /* z transforms (y_to_x, x_to_y): kx lines a block transforms */
   int32_t x_rows_per_block;   /* x pass (dft_x_realspace): z rows a block takes */

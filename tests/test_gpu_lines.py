@@ -1,0 +1,52 @@
+"""The line solver of the per-mode solves (line_solver.cu) and the mean lines (k_mean) at the sizes where
+they can go wrong, against the numpy oracle: the smallest ny that a spline order takes (the first and last
+rows' wide profiles overlap), the edges of the staged chunks (ny = bw + 24 c and one more), even ny, mode
+counts that are no multiple of a tile, every band width in use, one and two scalars, control, both time
+step rules and both precisions.  Tolerances: FP64 1e-11 of the field as the other trajectory tests,
+mixed 1e-5."""
+import numpy as np
+import pytest
+
+from channel_passive_b200 import Channel
+from oracle import kmm as okmm
+from tests.helpers import STATE_SLOTS, STATE_SLOTS2, make_pair, oracle_ctrl, rel_l2, seeded_state, with_scalar2
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [  # labs_k, ny
+    (6, 18), (6, 19), (6, 28), (6, 29), (6, 52), (6, 77), (4, 10), (4, 26), (4, 51), (5, 14), (5, 40), (7, 18),
+    (7, 30), (8, 22), (8, 33), (10, 26), (10, 45)]
+
+
+def _compare(cfg, p, nsteps, tol, scalars=1):
+    ops = okmm.make_operators(p)
+    U = seeded_state(cfg, ops.y)
+    if scalars == 2:
+        U = with_scalar2(U, U[6] * 0.5)
+    RK = okmm.set_initial_data_uvw(U.copy(), ops, p)
+    Uo, RKo, dt = U.copy(), RK.copy(), 0.01
+    for _ in range(nsteps):
+        dt, sc = okmm.rk3_step(Uo, RKo, ops, p, dt, ctrl=oracle_ctrl(ops, p))
+    with Channel(cfg) as ch:
+        ch.set_initial_data_uvw(U, 0.01)
+        out = ch.step(nsteps)
+        Ug, RKg = ch.download_state(U.shape[0])
+    for s in STATE_SLOTS2 if scalars == 2 else STATE_SLOTS:
+        assert rel_l2(Ug[s], Uo[s]) < tol, s
+    assert rel_l2(RKg[: RKo.shape[0]], RKo) < 10 * tol
+    assert abs(out["dt"] - dt) <= tol * dt
+    assert abs(out["wall_shear_stress"] - sc.wall_shear_stress) <= 10 * tol * abs(sc.wall_shear_stress)
+
+
+@pytest.mark.parametrize("labs_k,ny", SIZES)
+def test_lines_match_oracle(labs_k, ny):
+    cfg, p = make_pair(nx=12, ny=ny, nz=18, control_amp=-0.7, fixed_dt=ny % 2, labs_k=labs_k)
+    p.labs_k = labs_k
+    _compare(cfg, p, 2, 1e-11)
+
+
+@pytest.mark.parametrize("ny", [33, 53])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_two_scalars_match_oracle(ny, precision):
+    cfg, p = make_pair(nx=16, ny=ny, nz=16, control_amp=-0.7, fixed_dt=0, precision=precision, n_scalar=2)
+    _compare(cfg, p, 2, 1e-5 if precision else 1e-11, scalars=2)

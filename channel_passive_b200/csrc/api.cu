@@ -600,7 +600,8 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   if ((rc = make_plans(*h))) return fail(rc);
   prepare_kernels(*h);
   {
-    const cudaError_t e = prepare_transforms2();
+    cudaError_t e = prepare_transforms2();
+    if (e == cudaSuccess) e = prepare_transforms3();
     if (e != cudaSuccess) {
       set_error(std::string("transform set-up failed: ") + cudaGetErrorString(e));
       return fail(KMM_ERR_CUDA);

@@ -18,8 +18,8 @@
 namespace kmm {
 
 // Twiddles exp(-i 2 pi t / M) of the register DFT sizes, filled by the host (api.cu).
-constexpr int kRegSizes[] = {2, 3, 4, 6, 8, 9, 12, 16, 18, 24, 32};
-constexpr int kNumRegSizes = 11;
+constexpr int kRegSizes[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 27, 32};
+constexpr int kNumRegSizes = 17;
 constexpr int reg_tw_offset(int M) {
   int off = 0;
   for (int i = 0; i < kNumRegSizes; ++i) {
@@ -28,14 +28,16 @@ constexpr int reg_tw_offset(int M) {
   }
   return -1;
 }
-constexpr int kRegTwTotal = 2 + 3 + 4 + 6 + 8 + 9 + 12 + 16 + 18 + 24 + 32;
-// Defined in the one translation unit that includes this header (transforms2.cu).  The float2
+constexpr int kRegTwTotal = 2 + 3 + 4 + 5 + 6 + 8 + 9 + 10 + 12 + 15 + 16 + 18 + 20 + 24 + 25 + 27 + 32;
+// Each translation unit that includes this header has its own copy (fill_regtw).  The float2
 // copy lets FP32 DFTs take their twiddles as constant operands without conversions.
-__constant__ double2 c_regtw[kRegTwTotal];
-__constant__ float2 c_regtw32[kRegTwTotal];
+static __constant__ double2 c_regtw[kRegTwTotal];
+static __constant__ float2 c_regtw32[kRegTwTotal];
 
-// First radix of the Stockham factorisation of M (4s first, then 2, then 3).
-constexpr int first_radix(int M) { return (M % 4 == 0 && M != 8 && M != 32) || M == 4 ? 4 : (M % 2 == 0 ? 2 : 3); }
+// First radix of the Stockham factorisation of M (4s first, then 2, then 3, then 5).
+constexpr int first_radix(int M) {
+  return (M % 4 == 0 && M != 8 && M != 32) || M == 4 ? 4 : M % 2 == 0 ? 2 : M % 3 == 0 ? 3 : 5;
+}
 
 template <typename C, int M>
 __device__ __forceinline__ C twr(int t, int sign) {
@@ -63,17 +65,38 @@ __device__ __forceinline__ void stockham_pass(const C (&in)[M], C (&out)[M], int
       a[p] = in[idx + p * Q];
       if (p > 0 && k > 0) a[p] = cmul(a[p], twr<C, M>((p * k * (M / (Ns * R))) % M, sign));
     }
-    if (R == 2) {
+    if constexpr (R == 2) {
       const C x0 = a[0], x1 = a[1];
       a[0] = cadd(x0, x1);
       a[1] = csub(x0, x1);
-    } else if (R == 4) {
+    } else if constexpr (R == 4) {
       const C s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]), s13 = cadd(a[1], a[3]);
       const C d13 = cmul_si(csub(a[1], a[3]), sign);
       a[0] = cadd(s02, s13);
       a[2] = csub(s02, s13);
       a[1] = cadd(d02, d13);
       a[3] = csub(d02, d13);
+    } else if constexpr (R == 5) {
+      // with s = sin, c = cos of 2 pi / 5 and 4 pi / 5: X1, X4 = m1 +- q1, X2, X3 = m2 +- q2
+      using R_t = decltype(a[0].x);
+      const R_t c1 = (R_t)0.30901699437494742410, c2 = (R_t)-0.80901699437494742410;
+      const R_t s1 = (R_t)0.95105651629515357212, s2 = (R_t)0.58778525229247312917;
+      const C a0 = a[0], p1 = cadd(a[1], a[4]), p2 = cadd(a[2], a[3]), d1 = csub(a[1], a[4]), d2 = csub(a[2], a[3]);
+      C m1, m2, e1, e2;
+      m1.x = a0.x + c1 * p1.x + c2 * p2.x;
+      m1.y = a0.y + c1 * p1.y + c2 * p2.y;
+      m2.x = a0.x + c2 * p1.x + c1 * p2.x;
+      m2.y = a0.y + c2 * p1.y + c1 * p2.y;
+      e1.x = s1 * d1.x + s2 * d2.x;
+      e1.y = s1 * d1.y + s2 * d2.y;
+      e2.x = s2 * d1.x - s1 * d2.x;
+      e2.y = s2 * d1.y - s1 * d2.y;
+      const C q1 = cmul_si(e1, sign), q2 = cmul_si(e2, sign);
+      a[0] = cadd(a0, cadd(p1, p2));
+      a[1] = cadd(m1, q1);
+      a[4] = csub(m1, q1);
+      a[2] = cadd(m2, q2);
+      a[3] = csub(m2, q2);
     } else {  // R == 3
       using R_t = decltype(a[0].x);
       const R_t h = (R_t)0.86602540378443864676;  // sin(2 pi / 3)

@@ -259,6 +259,12 @@ int xphys2_row_blocks(const Handle &h);
 cudaError_t launch_xadj2(Handle &h, const double2 *base_mid, double2 *lmid, double scale, cudaStream_t st);
 cudaError_t launch_zfwd2(Handle &h, const void *mid, void *dst_planes, int nfield, double scale,
                          bool dst_fp64, cudaStream_t st, bool fp64 = false);
+// The same kernels for the other common lengths, for the step with one scalar (transforms3.cu).
+cudaError_t prepare_transforms3();
+cudaError_t launch_zinv3(Handle &h, const double2 *src_planes, void *mid, int nfield, cudaStream_t st, bool fp64);
+cudaError_t launch_xphys3(Handle &h, void *mid, int substep, cudaStream_t st);
+cudaError_t launch_zfwd3(Handle &h, const void *mid, void *dst_planes, int nfield, double scale, bool dst_fp64,
+                         cudaStream_t st, bool fp64);
 // Per-mode solves of one substep (wavespace_split.cu): hvhg, Helmholtz and assembly kernels on
 // st, the mean lines on h.side (joined back to st before return).
 cudaError_t launch_wavespace_split(Handle &h, int substep, const double *dt_override, cudaStream_t st);

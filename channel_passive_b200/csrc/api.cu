@@ -281,7 +281,7 @@ int check_device_error(Handle &h, int err) {
   KMM_CUDA(cudaMemcpy(&h.dsc->err, &zero, sizeof(int), cudaMemcpyHostToDevice));
   if (err == KMM_ERR_DT) set_error("ABORT due to timestep dt (dt <= 1e-14 or dt > 1e5)");
   else if (err == KMM_ERR_NONFINITE) set_error("non-finite velocity in the physical-space step");
-  else if (err == KMM_ERR_TIMEOUT) set_error("a bounded device wait gave up: a TMA tile copy of the z transforms did not complete");
+  else if (err == KMM_ERR_TIMEOUT) set_error("a bounded device wait gave up: a staged copy (z transforms, line solver) did not complete");
   else set_error("device error " + std::to_string(err));
   return err;
 }

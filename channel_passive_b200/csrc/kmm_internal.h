@@ -312,6 +312,7 @@ int64_t vop_factor_doubles(const Handle &h);
 bool line_solver_fits(Handle &h);
 int64_t tile_factor_doubles(const Handle &h);
 cudaError_t prepare_line_solver(Handle &h, cudaStream_t st);
+cudaError_t launch_line_hvhg(Handle &h, int substep, cudaStream_t st);
 cudaError_t launch_line_factor(Handle &h, int substep, const double *dt_ptr, cudaStream_t st);
 cudaError_t launch_line_solver(Handle &h, int substep, const double *dt_ptr, cudaStream_t st);
 // Whether the handle can cache the Helmholtz factors: a fixed time step and one scalar.

@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
   constexpr int LR = 2;  // rows whose loads a thread has in flight together
   for (int rb = rt; rb < n; rb += LR * RT) {
     double2 st[LR][NST], d2[LR][NST];
-    PT hh[LR][7];
+    PT hh[LR][4];
 #pragma unroll
     for (int q = 0; q < LR; ++q) {
       const int o = min(rb + q * RT, n - 1) * nm + ml;
@@ -195,9 +195,10 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
         st[q][i] = ld_stream(a.RK[store_of[i]] + o);
         if (s == 1) d2[q][i] = ld_stream(reinterpret_cast<const double2 *>(a.hl[d2_of[i]]) + o);
       }
-#pragma unroll
-      for (int i = H_HV0; i <= H_V3; ++i) hh[q][i] = ld_stream(hp(i) + o);
-      if constexpr (NS == 2) hh[q][6] = ld_stream(hp(H_HT2) + o);
+      hh[q][0] = ld_stream(hp(H_HT) + o);
+      hh[q][1] = ld_stream(hp(H_G2) + o);
+      hh[q][2] = ld_stream(hp(H_HV0) + o);
+      if constexpr (NS == 2) hh[q][3] = ld_stream(hp(H_HT2) + o);
     }
 #pragma unroll
     for (int q = 0; q < LR; ++q) {
@@ -205,8 +206,7 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
       if (r >= n) break;
       const bool in = live && r > 0 && r < n - 1;
       auto wide = [&](int i) { return z2((double)hh[q][i].x, (double)hh[q][i].y); };
-      const double2 h[4] = {wide(H_HT), zadd(wide(H_G2), wide(H_G3)),
-                            zadd(wide(H_HV0), zadd(wide(H_V2), wide(H_V3))), NS == 2 ? wide(6) : z2(0.0, 0.0)};
+      const double2 h[4] = {wide(0), wide(1), wide(2), NS == 2 ? wide(3) : z2(0.0, 0.0)};
       double *x = pl + r * kTile + k;
 #pragma unroll
       for (int i = 0; i < NST; ++i) {
@@ -427,22 +427,19 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
     const int o[2] = {r0 * nm + ml, (n - 1 - r0) * nm + ml};
     double2 hv[2], hg[2];  // the nonlinear terms, on their way while the operator rows arrive
     {
-      PT q[2][5];
+      PT q[2][2];
 #pragma unroll
       for (int w = 0; w < 2; ++w)
         if (s != 3) {
           q[w][0] = ld_stream(hp(H_HV0) + o[w]);
-          q[w][1] = ld_stream(hp(H_V2) + o[w]);
-          q[w][2] = ld_stream(hp(H_V3) + o[w]);
-          q[w][3] = ld_stream(hp(H_G2) + o[w]);
-          q[w][4] = ld_stream(hp(H_G3) + o[w]);
+          q[w][1] = ld_stream(hp(H_G2) + o[w]);
         }
       ok = mbar_wait_bounded(rowb, (p0 / per) & 1);
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
         auto wide = [&](int i) { return z2((double)q[w][i].x, (double)q[w][i].y); };
-        hv[w] = s == 3 ? z2(0.0, 0.0) : zadd(wide(0), zadd(wide(1), wide(2)));
-        hg[w] = s == 3 ? z2(0.0, 0.0) : zadd(wide(3), wide(4));
+        hv[w] = s == 3 ? z2(0.0, 0.0) : wide(0);
+        hg[w] = s == 3 ? z2(0.0, 0.0) : wide(1);
       }
     }
     if (__syncthreads_or(!ok)) {
@@ -526,6 +523,153 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// k_line_hvhg: hvhg.f90:56-159 for a tile of modes, the lines in shared memory as in k_lines (the D0
+// factor is the same for all modes and read through L1):
+//   h_v = i k2 (kx f2 + kz f4) + D1 c(a3) + D2 c(i kz f4 + i kx f2),  a3 = -kx^2 f1 - 2 kx kz f5 - kz^2 f3
+//   h_g = kx kz (f1 - f3) + (kz^2 - kx^2) f5 + D1 c(i kx f4 - i kz f2)
+//   h_theta = -(i kx f7 + i kz f9 + D1 c(f8)), with c(f) = D0^{-1} f.
+// At substep 1 also D2 D0^{-1} of the RK stores, and the control probes v(+-y_d) = w . v of the
+// substep's starting v.  k_hvhg (wavespace_split.cu) takes 77 us on 64x65x64 FP64, 37 us even on 16x33x16.
+struct HvhgArgs {
+  int n, nxh, nz, substep, nmodes;
+  const void *P[11];
+  const double2 *RK[4], *v;
+  void *hl[H_COUNT];
+  const double *l0, *u0, *tt, *wlo, *whi;
+  double2 *vwall;
+  double control_amp, lmfxr, lmfzr;
+  DevScalars *dsc;
+};
+
+template <typename PT> __device__ __forceinline__ PT narrow(double2 v);
+template <> __device__ __forceinline__ double2 narrow<double2>(double2 v) { return v; }
+template <> __device__ __forceinline__ float2 narrow<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
+
+template <int BW, typename PT, int NS>
+__global__ void __launch_bounds__(kHelmThreads, 3) k_line_hvhg(HvhgArgs a) {
+  extern __shared__ __align__(16) double hvhg_lines[];
+  if (a.dsc->err) return;
+  constexpr int RT = kHelmThreads / kTile;
+  const int n = a.n, s = a.substep, tid = threadIdx.x, nm = a.nmodes, ps = (n | 1) * kTile;
+  const int k = tid % kTile, rt = tid / kTile, m = blockIdx.x * kTile + k;
+  const bool live = m > 0 && m < nm;
+  const int ml = live ? m : 0;
+  const ModeK kk = mode_k(ml, a.nxh, a.nz, a.lmfxr, a.lmfzr);
+  const double kx = kk.kx, kz = kk.kz, k2 = kk.k2;
+  double *pl = hvhg_lines;
+  auto prod = [&](int i, int o) {
+    const PT v = ld_stream(reinterpret_cast<const PT *>(a.P[i]) + o);
+    return z2((double)v.x, (double)v.y);
+  };
+  auto put = [&](int plane, int r, double2 v) {
+    pl[plane * ps + r * kTile + k] = v.x;
+    pl[(plane + 1) * ps + r * kTile + k] = v.y;
+  };
+#pragma unroll 2
+  for (int r = rt; r < n; r += RT) {
+    const int o = r * nm + ml;
+    const double2 f1 = prod(0, o), f2 = prod(1, o), f3 = prod(2, o), f4 = prod(3, o), f5 = prod(4, o);
+    put(0, r, zsub(zsub(zscale(-kx * kx, f1), zscale(2.0 * kx * kz, f5)), zscale(kz * kz, f3)));
+    put(2, r, prod(6, o));
+    put(4, r, z2(kz * f2.y - kx * f4.y, kx * f4.x - kz * f2.x));
+    put(6, r, z2(-kz * f4.y - kx * f2.y, kz * f4.x + kx * f2.x));
+    if constexpr (NS == 2) put(8, r, prod(9, o));
+  }
+  __syncthreads();
+  // c = D0^{-1} of the first `planes` planes, in place, a thread per plane and mode
+  auto solve = [&](int planes) {
+    if (rt < planes) {
+      double *x = pl + rt * ps + k;
+      const double *l0 = a.l0, *u0 = a.u0;
+      fixed_fwd<BW, kTile>(x, n, [&](int r, int d) { return l0[r * (2 * BW + 1) + d] * l0[r * (2 * BW + 1)]; },
+                           [&](int r) { return l0[r * (2 * BW + 1)]; });
+      fixed_bwd<BW, kTile>(x, n, [&](int r, int e) { return u0[r * 2 * BW + e - 1]; });
+    }
+    __syncthreads();
+  };
+  // row r of D_d times the coefficients of a plane pair
+  auto dot = [&](const double *tt, int d, int plane, int r) {
+    const double *x = pl + plane * ps + first_col<BW>(r, n) * kTile + k;
+    double2 acc = z2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j <= 2 * BW; ++j) {
+      const double e = tt[3 * j + d];
+      acc.x += e * x[j * kTile];
+      acc.y += e * x[ps + j * kTile];
+    }
+    return acc;
+  };
+  solve(NS == 2 ? 10 : 8);
+  for (int r = rt; r < n; r += RT) {
+    const int o = r * nm + ml;
+    const double *tt = row_entries<BW>(a.tt, r);
+    const double2 f1 = prod(0, o), f2 = prod(1, o), f3 = prod(2, o), f4 = prod(3, o), f5 = prod(4, o);
+    const double2 f7 = prod(5, o), f9 = prod(7, o);
+    const double2 hv = zadd(z2(-k2 * (kx * f2.y + kz * f4.y), k2 * (kx * f2.x + kz * f4.x)),
+                            zadd(dot(tt, 1, 0, r), dot(tt, 2, 6, r)));
+    const double2 hg = zadd(zadd(zscale(kx * kz, zsub(f1, f3)), zscale(kz * kz - kx * kx, f5)), dot(tt, 1, 4, r));
+    const double2 t8 = dot(tt, 1, 2, r);
+    if (live) {
+      reinterpret_cast<PT *>(a.hl[H_HV0])[o] = narrow<PT>(hv);
+      reinterpret_cast<PT *>(a.hl[H_G2])[o] = narrow<PT>(hg);
+      reinterpret_cast<PT *>(a.hl[H_HT])[o] =
+          narrow<PT>(z2(kx * f7.y + kz * f9.y - t8.x, -(kx * f7.x + kz * f9.x + t8.y)));
+    }
+    if constexpr (NS == 2) {
+      const double2 p = prod(8, o), q = prod(10, o), t = dot(tt, 1, 8, r);
+      if (live)
+        reinterpret_cast<PT *>(a.hl[H_HT2])[o] = narrow<PT>(z2(kx * p.y + kz * q.y - t.x, -(kx * p.x + kz * q.x + t.y)));
+    }
+  }
+  if (s == 1) {
+    __syncthreads();
+    constexpr int NST = 2 + NS, store_of[4] = {1, 2, 0, 3}, line_of[4] = {H_DP, H_DT, H_DG, H_DT2};
+    for (int r = rt; r < n; r += RT)
+#pragma unroll
+      for (int i = 0; i < NST; ++i) put(2 * i, r, ld_stream(a.RK[store_of[i]] + r * nm + ml));
+    __syncthreads();
+    solve(2 * NST);
+    for (int r = rt; r < n; r += RT) {
+      const double *tt = row_entries<BW>(a.tt, r);
+#pragma unroll
+      for (int i = 0; i < NST; ++i) {
+        const double2 d2 = dot(tt, 2, 2 * i, r);
+        if (live) reinterpret_cast<double2 *>(a.hl[line_of[i]])[r * nm + m] = d2;
+      }
+    }
+  }
+  if (a.control_amp != 0.0) {  // (uniform) the control probes, summed over rt in order
+    double2 lo = z2(0.0, 0.0), hi = lo;
+    for (int r = rt; r < n; r += RT) {
+      const double2 v = ld_stream(a.v + r * nm + ml);
+      lo = zadd(lo, zscale(__ldg(a.wlo + r), v));
+      hi = zadd(hi, zscale(__ldg(a.whi + r), v));
+    }
+    __syncthreads();  // the planes are free
+    double *red = pl + tid * 4;
+    red[0] = lo.x;
+    red[1] = lo.y;
+    red[2] = hi.x;
+    red[3] = hi.y;
+    __syncthreads();
+    if (tid < kTile && live) {
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int q = 0; q < RT; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] += pl[(q * kTile + tid) * 4 + i];
+      a.vwall[m] = z2(acc[0], acc[1]);
+      a.vwall[nm + m] = z2(acc[2], acc[3]);
+    }
+  }
+}
+
+// Shared memory of k_line_hvhg: its planes, and at least the probes' sums.
+size_t line_hvhg_bytes(const Handle &h) {
+  const size_t planes = (size_t)(h.nsc == 2 ? 10 : 8) * (size_t)(h.ny | 1) * kTile;
+  return sizeof(double) * (planes > 4 * kHelmThreads ? planes : 4 * kHelmThreads);
+}
+
 int smem_attr(cudaDeviceAttr attr) {
   int dev = 0, v = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, attr, dev) != cudaSuccess) return 0;
@@ -592,6 +736,42 @@ cudaError_t helm_bw(Handle &h, int substep, const double *dt_ptr, cudaStream_t s
 }
 
 template <int BW>
+cudaError_t hvhg_bw(Handle &h, int substep, cudaStream_t st) {
+  const OpsOffsets off = ops_offsets(h.bw, h.ny);
+  HvhgArgs a{};
+  a.n = h.ny;
+  a.nxh = h.nxh;
+  a.nz = h.nz;
+  a.substep = substep;
+  a.nmodes = (int)h.nmodes;
+  for (int i = 0; i < 5 + 3 * h.nsc; ++i)
+    a.P[i] = h.mixed ? (const void *)(reinterpret_cast<const float2 *>(h.P) + i * h.ns)
+                     : reinterpret_cast<const double2 *>(h.P) + i * h.ns;
+  const HelmArgs l = helm_args(h, substep, nullptr);
+  for (int i = 0; i < 4; ++i) a.RK[i] = l.RK[i];
+  a.v = l.S[1];
+  for (int i = 0; i < H_COUNT; ++i) a.hl[i] = const_cast<void *>(l.hl[i]);
+  const int64_t tw = (int64_t)h.ny * (4 * BW + 1);
+  a.l0 = h.dops + off.t0 + 3 * tw;
+  a.u0 = a.l0 + (int64_t)h.ny * (2 * BW + 1);
+  a.tt = h.dops + off.tt;
+  a.wlo = h.dops + off.wlo;
+  a.whi = h.dops + off.whi;
+  a.vwall = h.vwall;
+  a.control_amp = h.cfg.control_amp;
+  a.lmfxr = h.lmfxr;
+  a.lmfzr = h.lmfzr;
+  a.dsc = h.dsc;
+  const unsigned tiles = (unsigned)((h.nmodes + kTile - 1) / kTile);
+  const size_t bytes = line_hvhg_bytes(h);
+  if (h.mixed && h.nsc == 2) k_line_hvhg<BW, float2, 2><<<tiles, kHelmThreads, bytes, st>>>(a);
+  else if (h.mixed) k_line_hvhg<BW, float2, 1><<<tiles, kHelmThreads, bytes, st>>>(a);
+  else if (h.nsc == 2) k_line_hvhg<BW, double2, 2><<<tiles, kHelmThreads, bytes, st>>>(a);
+  else k_line_hvhg<BW, double2, 1><<<tiles, kHelmThreads, bytes, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int BW>
 cudaError_t factor_bw(Handle &h, int substep, const double *dt_ptr, cudaStream_t st) {
   const HelmArgs a = helm_args(h, substep, dt_ptr);
   k_line_factor<BW><<<dim3((unsigned)((h.nmodes + 31) / 32), (unsigned)(1 + h.nsc)), 32, 0, st>>>(a);
@@ -605,6 +785,10 @@ cudaError_t prepare_bw(Handle &h, cudaStream_t st) {
   };
   cudaError_t e = lim(k_lines<BW, float2, 1>);
   if (e == cudaSuccess) e = lim(k_lines<BW, double2, 1>);
+  if (e == cudaSuccess) e = lim(k_line_hvhg<BW, float2, 1>);
+  if (e == cudaSuccess) e = lim(k_line_hvhg<BW, double2, 1>);
+  if (e == cudaSuccess) e = lim(k_line_hvhg<BW, float2, 2>);
+  if (e == cudaSuccess) e = lim(k_line_hvhg<BW, double2, 2>);
   if (e == cudaSuccess) e = lim(k_lines<BW, float2, 2>);
   if (e == cudaSuccess) e = lim(k_lines<BW, double2, 2>);
   if (e != cudaSuccess) return e;
@@ -654,6 +838,10 @@ int64_t tile_factor_doubles(const Handle &h) {
 
 cudaError_t prepare_line_solver(Handle &h, cudaStream_t st) {
   return with_bw(h.bw, [&]<int BW>() { return prepare_bw<BW>(h, st); });
+}
+
+cudaError_t launch_line_hvhg(Handle &h, int substep, cudaStream_t st) {
+  return with_bw(h.bw, [&]<int BW>() { return hvhg_bw<BW>(h, substep, st); });
 }
 
 cudaError_t launch_line_factor(Handle &h, int substep, const double *dt_ptr, cudaStream_t st) {

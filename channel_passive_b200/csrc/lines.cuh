@@ -244,6 +244,73 @@ __device__ __forceinline__ void bwd_chunk(unsigned x, unsigned co, unsigned bx, 
   }
 }
 
+// Forward substitution in place over n values ST apart, right-looking, the factors shared by all modes: lf(r, d) = L(r, r-d) / L(r, r) for
+// d = 1..2BW, rp(r) = 1 / L(r, r).
+template <int BW, int ST, typename LF, typename RP>
+__device__ __forceinline__ void fixed_fwd(double *x, int n, LF lf, RP rp) {
+  constexpr int RB = 4;
+  double acc[BW];
+#pragma unroll
+  for (int k = 0; k < BW; ++k) acc[k] = x[k * ST] * rp(k);
+  int r = 0;
+  for (; r + RB + BW <= n - BW; r += RB) {
+    double b[RB], l[RB][BW], z[RB];
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+      b[i] = x[(r + i + BW) * ST] * rp(r + i + BW);
+#pragma unroll
+      for (int k = 1; k <= BW; ++k) l[i][k - 1] = lf(r + i + k, k);
+    }
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+      z[i] = acc[0];
+#pragma unroll
+      for (int k = 1; k < BW; ++k) acc[k - 1] = acc[k] - l[i][k - 1] * z[i];
+      acc[BW - 1] = b[i] - l[i][BW - 1] * z[i];
+    }
+#pragma unroll
+    for (int i = 0; i < RB; ++i) x[(r + i) * ST] = z[i];
+  }
+  for (; r < n; ++r) {  // the rows near the end, which reach 2BW rows back
+    double t = x[r * ST] * rp(r);
+    for (int d = min(r, r >= n - BW ? 2 * BW : BW); d >= 1; --d) t -= lf(r, d) * x[(r - d) * ST];
+    x[r * ST] = t;
+  }
+}
+
+// Backward substitution: uf(r, e) = U(r, r+e), e = 1..2BW.
+template <int BW, int ST, typename UF>
+__device__ __forceinline__ void fixed_bwd(double *x, int n, UF uf) {
+  constexpr int RB = 4;
+  double acc[BW];
+#pragma unroll
+  for (int k = 0; k < BW; ++k) acc[k] = x[(n - 1 - k) * ST];
+  int r = n - 1;
+  for (; r - RB - BW + 1 >= BW; r -= RB) {
+    double b[RB], u[RB][BW], z[RB];
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+      b[i] = x[(r - i - BW) * ST];
+#pragma unroll
+      for (int k = 1; k <= BW; ++k) u[i][k - 1] = uf(r - i - k, k);
+    }
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+      z[i] = acc[0];
+#pragma unroll
+      for (int k = 1; k < BW; ++k) acc[k - 1] = acc[k] - u[i][k - 1] * z[i];
+      acc[BW - 1] = b[i] - u[i][BW - 1] * z[i];
+    }
+#pragma unroll
+    for (int i = 0; i < RB; ++i) x[(r - i) * ST] = z[i];
+  }
+  for (; r >= 0; --r) {
+    double t = x[r * ST];
+    for (int e = min(n - 1 - r, r < BW ? 2 * BW : BW); e >= 1; --e) t -= uf(r, e) * x[(r + e) * ST];
+    x[r * ST] = t;
+  }
+}
+
 // Row r of an operator spans 2BW+1 columns from here (the near-boundary packing of the first and
 // last BW rows, LABS_full_to_band, module_labs.f90:301-328).
 template <int BW>
@@ -331,7 +398,9 @@ __device__ __forceinline__ void vrow(const Tabs<BW> &tb, int r, int n, double k2
   for (int e = -2 * BW; e <= 2 * BW; ++e) row[e + 2 * BW] = -k2 * r0[e] + r2[e];
 }
 
-// Lines k_hvhg hands to k_helmholtz.  The six nonlinear-term lines H_HV0..H_V3 are combinations
+// Lines hvhg hands to the Helmholtz solves.  (The line solver's k_line_hvhg fills H_HV0 with all of h_v
+// and H_G2 with all of h_g, and leaves H_V2, H_V3 and H_G3.)
+// k_hvhg's:  The six nonlinear-term lines H_HV0..H_V3 are combinations
 // of the products and are stored at the products' precision PT (float2 in the mixed path, packed
 // at (PT *)hl + i * ns); the substep-1 lines H_DP, H_DT, H_DG (D2 D0^{-1} of the FP64 RK stores)
 // stay double2 at hl + i * ns.

@@ -49,73 +49,6 @@ __host__ __device__ constexpr int64_t mean_line_doubles(int bw, int n) {
   return (int64_t)n * (8 + 2 * bw + 1) + 2 * bw * bw;
 }
 
-// Forward substitution in place over x[0..n), right-looking (lines.cuh): lf(r, d) = L(r, r-d) / L(r, r) for
-// d = 1..2BW, rp(r) = 1 / L(r, r).
-template <int BW, typename LF, typename RP>
-__device__ __forceinline__ void mean_fwd(double *x, int n, LF lf, RP rp) {
-  constexpr int RB = 4;
-  double acc[BW];
-#pragma unroll
-  for (int k = 0; k < BW; ++k) acc[k] = x[k] * rp(k);
-  int r = 0;
-  for (; r + RB + BW <= n - BW; r += RB) {
-    double b[RB], l[RB][BW], z[RB];
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      b[i] = x[r + i + BW] * rp(r + i + BW);
-#pragma unroll
-      for (int k = 1; k <= BW; ++k) l[i][k - 1] = lf(r + i + k, k);
-    }
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      z[i] = acc[0];
-#pragma unroll
-      for (int k = 1; k < BW; ++k) acc[k - 1] = acc[k] - l[i][k - 1] * z[i];
-      acc[BW - 1] = b[i] - l[i][BW - 1] * z[i];
-    }
-#pragma unroll
-    for (int i = 0; i < RB; ++i) x[r + i] = z[i];
-  }
-  for (; r < n; ++r) {  // the rows near the end, which reach 2BW rows back
-    double t = x[r] * rp(r);
-    for (int d = min(r, r >= n - BW ? 2 * BW : BW); d >= 1; --d) t -= lf(r, d) * x[r - d];
-    x[r] = t;
-  }
-}
-
-// Backward substitution: uf(r, e) = U(r, r+e), e = 1..2BW.
-template <int BW, typename UF>
-__device__ __forceinline__ void mean_bwd(double *x, int n, UF uf) {
-  constexpr int RB = 4;
-  double acc[BW];
-#pragma unroll
-  for (int k = 0; k < BW; ++k) acc[k] = x[n - 1 - k];
-  int r = n - 1;
-  for (; r - RB - BW + 1 >= BW; r -= RB) {
-    double b[RB], u[RB][BW], z[RB];
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      b[i] = x[r - i - BW];
-#pragma unroll
-      for (int k = 1; k <= BW; ++k) u[i][k - 1] = uf(r - i - k, k);
-    }
-#pragma unroll
-    for (int i = 0; i < RB; ++i) {
-      z[i] = acc[0];
-#pragma unroll
-      for (int k = 1; k < BW; ++k) acc[k - 1] = acc[k] - u[i][k - 1] * z[i];
-      acc[BW - 1] = b[i] - u[i][BW - 1] * z[i];
-    }
-#pragma unroll
-    for (int i = 0; i < RB; ++i) x[r - i] = z[i];
-  }
-  for (; r >= 0; --r) {
-    double t = x[r];
-    for (int e = min(n - 1 - r, r < BW ? 2 * BW : BW); e >= 1; --e) t -= uf(r, e) * x[r + e];
-    x[r] = t;
-  }
-}
-
 template <int BW, bool SM>
 __global__ void __launch_bounds__(256) k_mean(MeanArgs a) {
   extern __shared__ double mean_smem[];
@@ -185,9 +118,9 @@ __global__ void __launch_bounds__(256) k_mean(MeanArgs a) {
     // D0 solves: the flux product (and the store at substep 1)
     if (lane < (s == 1 ? 4 : 2)) {
       double *x = F + lane * n;
-      mean_fwd<BW>(x, n, [&](int r, int d) { return tb.l0[r * (2 * BW + 1) + d] * tb.l0[r * (2 * BW + 1)]; },
+      fixed_fwd<BW, 1>(x, n, [&](int r, int d) { return tb.l0[r * (2 * BW + 1) + d] * tb.l0[r * (2 * BW + 1)]; },
                    [&](int r) { return tb.l0[r * (2 * BW + 1)]; });
-      mean_bwd<BW>(x, n, [&](int r, int e) { return tb.u0[r * 2 * BW + e - 1]; });
+      fixed_bwd<BW, 1>(x, n, [&](int r, int e) { return tb.u0[r * 2 * BW + e - 1]; });
     }
     __syncwarp();
     const double gamma = dt * rkc(3, s), alpha = dt * rkc(1, s) * visc;
@@ -208,12 +141,12 @@ __global__ void __launch_bounds__(256) k_mean(MeanArgs a) {
   if (warp >= 4 || !mine) return;
   if (lane < 2) {
     double *x = R + lane * n;
-    mean_fwd<BW>(x, n,
+    fixed_fwd<BW, 1>(x, n,
                  [&](int r, int d) {
                    return d <= BW ? lu.l[r * (BW + 1) + d] : lu.lx[(r - (n - BW)) * BW + d - BW - 1];
                  },
                  [&](int r) { return lu.l[r * (BW + 1)]; });
-    mean_bwd<BW>(x, n, [&](int r, int e) { return e <= BW ? lu.u[r * BW + e - 1] : lu.ux[r * BW + e - BW - 1]; });
+    fixed_bwd<BW, 1>(x, n, [&](int r, int e) { return e <= BW ? lu.u[r * BW + e - 1] : lu.ux[r * BW + e - BW - 1]; });
   }
   __syncwarp();
   // LABS_integration of the coefficients, real and imaginary part

@@ -835,6 +835,7 @@ cudaError_t split_bw(Handle &h, int part, int substep, const double *dt_ptr, cud
     if ((e = cudaStreamWaitEvent(h.side, h.ev_fork, 0)) != cudaSuccess) return e;
     if ((e = launch_mean(h, substep, dtp, h.side)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(h.ev_join, h.side)) != cudaSuccess) return e;
+    if (h.lines) return launch_line_hvhg(h, substep, st);
     if (h.nsc == 2) {
       if (h.mixed) k_hvhg<BW, float2, 2><<<blocks, kLanes * (kRoles + 1), tsm, st>>>(a);
       else k_hvhg<BW, double2, 2><<<blocks, kLanes * (kRoles + 1), tsm, st>>>(a);

@@ -35,7 +35,8 @@ extern "C" {
 #define KMM_ERR_DT 3          /* dt <= 1e-14 or dt > 1e5 (dft_x_realspace.f90:494-497) */
 #define KMM_ERR_NONFINITE 4   /* NaN / Inf in the velocity maximum or in uploaded state */
 #define KMM_ERR_ARG 5         /* null pointer, bad substep, size mismatch */
-#define KMM_ERR_TIMEOUT 6     /* a bounded device wait gave up (a TMA tile copy of the z transforms) */
+#define KMM_ERR_TIMEOUT 6     /* a bounded device wait gave up (a TMA tile copy of the z transforms, a bulk
+                                 copy of the line solver) */
 #define KMM_ERR_IO 7          /* checkpoint file: unreadable, missing dataset, unexpected shape or
                                  type (the checks of module_hdf5_io.f90:212-345, same messages) */
 
@@ -269,7 +270,8 @@ int kmm_set_tuning(kmm_handle *h, const kmm_tuning *t);
 #define KMM_K_ZFWD 4        /* x_to_y: z forward transform of the 8 products (+ rescale) */
 #define KMM_K_HVHG 5        /* wavespace part 1: control probe, mean-mode fork, hvhg D0 solves */
 #define KMM_K_HELMHOLTZ 6   /* wavespace part 2: theta, g, phi and v Helmholtz solves */
-#define KMM_K_ASSEMBLE 7    /* wavespace part 3: C1/C2 assembly, u and w (the join of the mean-mode
+#define KMM_K_ASSEMBLE 7    /* wavespace part 3: C1/C2 assembly, u and w (up to 12000 modes part of
+                               KMM_K_HELMHOLTZ, and nothing here; the join of the mean-mode
                                lines, which run beside the solver kernels, is outside every id) */
 
 /* Runs nsteps RK3 steps launching kernel by kernel with a CUDA event pair around every

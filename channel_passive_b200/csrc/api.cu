@@ -601,7 +601,7 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   prepare_kernels(*h);
   {
     cudaError_t e = prepare_transforms2();
-    if (e == cudaSuccess) e = prepare_transforms3();
+    if (e == cudaSuccess) e = prepare_transforms3(*h);
     if (e != cudaSuccess) {
       set_error(std::string("transform set-up failed: ") + cudaGetErrorString(e));
       return fail(KMM_ERR_CUDA);

@@ -260,7 +260,7 @@ cudaError_t launch_xadj2(Handle &h, const double2 *base_mid, double2 *lmid, doub
 cudaError_t launch_zfwd2(Handle &h, const void *mid, void *dst_planes, int nfield, double scale,
                          bool dst_fp64, cudaStream_t st, bool fp64 = false);
 // The same kernels for the other common lengths, for the step with one scalar (transforms3.cu).
-cudaError_t prepare_transforms3();
+cudaError_t prepare_transforms3(const Handle &h);
 cudaError_t launch_zinv3(Handle &h, const double2 *src_planes, void *mid, int nfield, cudaStream_t st, bool fp64);
 cudaError_t launch_xphys3(Handle &h, void *mid, int substep, cudaStream_t st);
 cudaError_t launch_zfwd3(Handle &h, const void *mid, void *dst_planes, int nfield, double scale, bool dst_fp64,

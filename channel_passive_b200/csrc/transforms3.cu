@@ -43,30 +43,27 @@ template <typename F> bool with_other_shape(int N, F &&f) {
     default: return false;
   }
 }
-constexpr int kOtherLengths[] = {27,  30,  45,  54,  60,  75,  81,  90,  108, 120, 135, 150, 162,
-                                 180, 216, 225, 240, 243, 270, 300, 324, 360, 375, 432, 480};
 
 }  // namespace
 
-cudaError_t prepare_transforms3() {
-  int dev = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e == cudaSuccess) e = fill_regtw();
-  if (e != cudaSuccess) return e;
-  for (int N : kOtherLengths)
-    with_other_shape(N, [&]<int N1, int N2>() {
-      using D = TCfg<double>;
-      using F = TCfg<float>;
-      set_smem(k_zinv2<double, N1, N2, D::KB>, optin);
-      set_smem(k_zinv2<float, N1, N2, F::KB>, optin);
-      set_smem(k_zfwd2<double, N1, N2, D::KB, double2>, optin);
-      set_smem(k_zfwd2<float, N1, N2, F::KB, float2>, optin);
-      set_smem(k_zfwd2<float, N1, N2, F::KB, double2>, optin);
-      set_smem(k_xphys2<double, N1, N2, D::ZB, D::ZT>, optin);
-      set_smem(k_xphys2<float, N1, N2, F::ZB, F::ZT>, optin);
-    });
-  return cudaSuccess;
+// Shared-memory limits of the kernels h's lengths use (setting all 25 lengths' took 1 ms of kmm_create).
+cudaError_t prepare_transforms3(const Handle &h) {
+  cudaError_t e = cudaSuccess;
+  using D = TCfg<double>;
+  using F = TCfg<float>;
+  bool used = with_other_shape(h.nz32, [&]<int N1, int N2>() {
+    set_smem(k_zinv2<double, N1, N2, D::KB>, h.smem_optin);
+    set_smem(k_zinv2<float, N1, N2, F::KB>, h.smem_optin);
+    set_smem(k_zfwd2<double, N1, N2, D::KB, double2>, h.smem_optin);
+    set_smem(k_zfwd2<float, N1, N2, F::KB, float2>, h.smem_optin);
+    set_smem(k_zfwd2<float, N1, N2, F::KB, double2>, h.smem_optin);
+  });
+  used |= with_other_shape(h.nx32, [&]<int N1, int N2>() {
+    set_smem(k_xphys2<double, N1, N2, D::ZB, D::ZT>, h.smem_optin);
+    set_smem(k_xphys2<float, N1, N2, F::ZB, F::ZT>, h.smem_optin);
+  });
+  if (used) e = fill_regtw();
+  return e;
 }
 
 // Each returns cudaErrorNotSupported for other lengths (the caller falls back).

@@ -574,8 +574,10 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
       if ((rc = dalloc(*h, &h->hdvh, 3 * (size_t)h->nmodes))) return fail(rc);
     }
     if ((rc = dalloc(*h, &h->fcdt, 3))) return fail(rc);
+    if ((rc = dalloc(*h, &h->fcount, 3))) return fail(rc);
     const double none[3] = {NAN, NAN, NAN};  // no dt cached yet
-    if (cudaMemcpy(h->fcdt, none, sizeof(none), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMemcpy(h->fcdt, none, sizeof(none), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemset(h->fcount, 0, 3 * sizeof(unsigned)) != cudaSuccess) {
       set_error("factor cache set-up failed");
       return fail(KMM_ERR_CUDA);
     }
@@ -647,7 +649,7 @@ int kmm_destroy(kmm_handle *hh) {
   adjoint_free(*h);
   void *ptrs[] = {h->S, h->RK, h->P, h->MID, h->dops, h->gains, h->vwall, h->zc,
                   h->ec, h->xr, h->ub, h->vf, h->dvw, h->w00, h->staging, h->stat,
-                  h->mid64, h->p64, h->hf, h->hinf, h->hdvh, h->fcdt, h->lf, h->lvf, h->fftpos, h->tw64, h->tw32, h->dsc};
+                  h->mid64, h->p64, h->hf, h->hinf, h->hdvh, h->fcdt, h->fcount, h->lf, h->lvf, h->fftpos, h->tw64, h->tw32, h->dsc};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (h->copy) cudaStreamSynchronize(h->copy);

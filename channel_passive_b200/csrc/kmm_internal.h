@@ -144,6 +144,7 @@ struct Handle {
   // the factor cache per substep and dt; and of v's.
   bool lines = false;                      // the Helmholtz solves run in line_solver.cu (line_solver_fits)
   double *lf = nullptr, *lvf = nullptr;
+  unsigned *fcount = nullptr;              // [substep] blocks of k_line_factor done (between launches 0)
   int smem_optin = 0, smem_sm = 0;         // the device's shared memory: most of a block, of an SM
   double *stat = nullptr;                  // statistics buffers (stat_layout), made on first use
   double2 *mid64 = nullptr, *p64 = nullptr;  // mixed handles: FP64 slab [6][nm] and products [6][ns]

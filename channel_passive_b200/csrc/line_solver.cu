@@ -33,6 +33,7 @@ struct HelmArgs {
   double *fac[3];           // TileFac sets of theta, of g and phi, and of a second scalar
   double *vf;               // of v
   double *fcdt;             // the dt the sets fac hold (a fixed time step), or null
+  unsigned *fcount;         // blocks of k_line_factor done with them
   bool cached;              // the sets may be kept while they hold this dt (Tuning::fcache)
   int stages;               // ring slots
 };
@@ -41,45 +42,56 @@ struct HelmArgs {
 // k_line_factor: one thread per mode and operator; op = blockIdx.y (0 theta, 1 g and phi, 2 theta2), or
 // v's operator with a.fac[0] null.  LuSweep's profile Crout LU, stored by tile.  A no-op while the
 // sets hold this dt (a fixed time step: 3 us against 0.5 ms once a substep and run).
+// The sets and the dt they hold are written here together, by the last block to finish: it runs beside the
+// transforms, and whatever becomes of the substep after it, the mark is that of the sets.  (For the same
+// reason it does not look at the error flag: some blocks would leave and others not.)
 template <int BW>
 __global__ void __launch_bounds__(32) k_line_factor(HelmArgs a) {
   const bool vop = a.fac[0] == nullptr;
-  if (!vop && (a.dsc->err || (a.cached && *a.fcdt == *a.dt_ptr))) return;
+  if (!vop && a.cached && *a.fcdt == *a.dt_ptr) return;
   const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= a.nmodes) return;
   const int n = a.n, op = blockIdx.y;
-  const Tabs<BW> tb = tabs_at<BW>(a.tabs, n);
-  const double k2 = mode_k((int)m, a.nxh, a.nz, a.lmfxr, a.lmfzr).k2;
-  double *f = (vop ? a.vf : a.fac[op]) + (m / kTile) * TileFac<BW>::size(n);
-  const int km = (int)(m % kTile);
-  double ca = 0.0, cb = 0.0;
-  if (!vop) {
-    cb = *a.dt_ptr * rkc(2, a.substep) * (op == 0 ? a.nu / a.pr : op == 1 ? a.nu : a.nu / a.pr2);
-    ca = 1.0 + cb * k2;
-  }
-  LuSweep<BW, 0, 0, true, TileU<BW>> lu;
-  lu.init(n, TileU<BW>{f + TileFac<BW>::bwd(n), f + TileFac<BW>::bx(n) + km, n, km});
-  const double2 bc[1] = {z2(0.0, 0.0)};
-  const double br[1] = {0.0};
-  double2 zc[1];
-  double zr[1];
-  for (int r = 1; r <= n; ++r) {
-    lu.step(r, [&](int rr, double *row, bool c) {
-      if (vop) vrow<BW>(tb, rr, n, k2, row, c);
-      else helm_row<BW>(tb, rr, n, ca, cb, row, c);
-    }, bc, br, zc, zr);
-    const int q = r - 1;  // 0-based
-    auto entry = [&](int row, int k) -> double & { return f[(int64_t)row * (BW + 1) * kTile + entry_at(BW + 1, k, km)]; };
-    if (q >= BW) entry(q - BW, 0) = lu.Lk[0];
-    else f[TileFac<BW>::fx(n) + (BW * BW + q) * kTile + km] = lu.Lk[0];
-#pragma unroll
-    for (int d = 1; d <= BW; ++d)
-      if (q >= d) entry(q - d, d) = lu.Lk[d] * lu.Lk[0];
-    if (q >= n - BW) {
-      double *x = f + TileFac<BW>::fx(n) + (q - (n - BW)) * BW * kTile + km;
-#pragma unroll
-      for (int d = BW + 1; d <= 2 * BW; ++d) x[(d - BW - 1) * kTile] = lu.Lk[d] * lu.Lk[0];
+  if (m < a.nmodes) {
+    const Tabs<BW> tb = tabs_at<BW>(a.tabs, n);
+    const double k2 = mode_k((int)m, a.nxh, a.nz, a.lmfxr, a.lmfzr).k2;
+    double *f = (vop ? a.vf : a.fac[op]) + (m / kTile) * TileFac<BW>::size(n);
+    const int km = (int)(m % kTile);
+    double ca = 0.0, cb = 0.0;
+    if (!vop) {
+      cb = *a.dt_ptr * rkc(2, a.substep) * (op == 0 ? a.nu / a.pr : op == 1 ? a.nu : a.nu / a.pr2);
+      ca = 1.0 + cb * k2;
     }
+    LuSweep<BW, 0, 0, true, TileU<BW>> lu;
+    lu.init(n, TileU<BW>{f + TileFac<BW>::bwd(n), f + TileFac<BW>::bx(n) + km, n, km});
+    const double2 bc[1] = {z2(0.0, 0.0)};
+    const double br[1] = {0.0};
+    double2 zc[1];
+    double zr[1];
+    for (int r = 1; r <= n; ++r) {
+      lu.step(r, [&](int rr, double *row, bool c) {
+        if (vop) vrow<BW>(tb, rr, n, k2, row, c);
+        else helm_row<BW>(tb, rr, n, ca, cb, row, c);
+      }, bc, br, zc, zr);
+      const int q = r - 1;  // 0-based
+      auto entry = [&](int row, int k) -> double & { return f[(int64_t)row * (BW + 1) * kTile + entry_at(BW + 1, k, km)]; };
+      if (q >= BW) entry(q - BW, 0) = lu.Lk[0];
+      else f[TileFac<BW>::fx(n) + (BW * BW + q) * kTile + km] = lu.Lk[0];
+#pragma unroll
+      for (int d = 1; d <= BW; ++d)
+        if (q >= d) entry(q - d, d) = lu.Lk[d] * lu.Lk[0];
+      if (q >= n - BW) {
+        double *x = f + TileFac<BW>::fx(n) + (q - (n - BW)) * BW * kTile + km;
+#pragma unroll
+        for (int d = BW + 1; d <= 2 * BW; ++d) x[(d - BW - 1) * kTile] = lu.Lk[d] * lu.Lk[0];
+      }
+    }
+  }
+  if (vop || !a.fcdt) return;
+  __syncwarp();
+  // every block has read the old mark by the time it counts
+  if (threadIdx.x == 0 && atomicAdd(a.fcount, 1u) + 1 == gridDim.x * gridDim.y) {
+    *a.fcount = 0;
+    *a.fcdt = *a.dt_ptr;
   }
 }
 
@@ -115,7 +127,6 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
   constexpr int NOP = L::NOP, NP = helm_planes(NS), CT = helm_chain_threads(NS);
   extern __shared__ __align__(128) double helm_smem[];
   if (a.dsc->err) return;  // a failed dt update leaves the state untouched (uniform over the block)
-  if (a.fcdt && blockIdx.x == 0 && threadIdx.x == 0) *a.fcdt = *a.dt_ptr;  // read by the next k_line_factor only
   const int n = a.n, s = a.substep, tid = threadIdx.x;
   const int nm = (int)a.nmodes, ps = L::plane(n);  // (a line has fewer than 2^31 elements)
   // outside the chains a thread works on one mode, in rows RT apart
@@ -710,6 +721,7 @@ HelmArgs helm_args(Handle &h, int substep, const double *dt_ptr) {
   const int at = h.fcdt ? nop * (substep - 1) : 0;
   for (int o = 0; o < nop; ++o) a.fac[o] = h.lf + (at + o) * set;
   a.fcdt = h.fcdt ? h.fcdt + (substep - 1) : nullptr;
+  a.fcount = h.fcount ? h.fcount + (substep - 1) : nullptr;
   a.cached = h.fcdt && h.tune.fcache;
   return a;
 }

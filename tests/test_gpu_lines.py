@@ -4,6 +4,8 @@ rows' wide profiles overlap), the edges of the staged chunks (ny = bw + 24 c and
 counts that are no multiple of a tile, every band width in use, one and two scalars, control, both time
 step rules and both precisions.  Tolerances: FP64 1e-11 of the field as the other trajectory tests,
 mixed 1e-5."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -50,3 +52,29 @@ def test_lines_match_oracle(labs_k, ny):
 def test_two_scalars_match_oracle(ny, precision):
     cfg, p = make_pair(nx=16, ny=ny, nz=16, control_amp=-0.7, fixed_dt=0, precision=precision, n_scalar=2)
     _compare(cfg, p, 2, 1e-5 if precision else 1e-11, scalars=2)
+
+
+def test_kept_factors_carry_their_own_time_step():
+    """A substep that ends between the factorisation and the solves (a device wait that gives up) leaves
+    the factors of its dt behind: a caller that goes back to the former dt gets that dt's operators.  The
+    factorisation alone is the internal launcher's (no public call ends there on purpose)."""
+    torch = pytest.importorskip("torch")
+    cfg, p = make_pair(nx=32, ny=33, nz=32, control_amp=-1.0)
+    U = seeded_state(cfg, okmm.make_operators(p).y)
+    out = []
+    for interrupted in (False, True):
+        with Channel(cfg) as ch:
+            ch.set_initial_data_uvw(U, 0.01)
+            ch.step(1)
+            if interrupted:
+                factor = getattr(ch._lib, "_ZN3kmm18launch_line_factorERNS_6HandleEiPKdP11CUstream_st")
+                factor.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
+                other = torch.tensor([0.02], dtype=torch.float64, device="cuda")
+                for s in (1, 2, 3):
+                    assert factor(ch._h, s, other.data_ptr(), None) == 0
+                torch.cuda.synchronize()
+            ch.step(1)
+            out.append(ch.download_state(10))
+    for f in STATE_SLOTS:
+        assert np.array_equal(out[0][0][f], out[1][0][f]), f
+    assert np.array_equal(out[0][1], out[1][1])

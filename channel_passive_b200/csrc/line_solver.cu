@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
   using L = HelmSmem<BW, NS>;
   constexpr int NOP = L::NOP, NP = helm_planes(NS), CT = helm_chain_threads(NS);
   extern __shared__ __align__(128) double helm_smem[];
-  if (a.dsc->err) return;  // a failed dt update leaves the state untouched (uniform over the block)
+  if (block_failed(a.dsc)) return;
   const int n = a.n, s = a.substep, tid = threadIdx.x;
   const int nm = (int)a.nmodes, ps = L::plane(n);  // (a line has fewer than 2^31 elements)
   // outside the chains a thread works on one mode, in rows RT apart
@@ -560,7 +560,7 @@ template <> __device__ __forceinline__ float2 narrow<float2>(double2 v) { return
 template <int BW, typename PT, int NS>
 __global__ void __launch_bounds__(kHelmThreads, 3) k_line_hvhg(HvhgArgs a) {
   extern __shared__ __align__(16) double hvhg_lines[];
-  if (a.dsc->err) return;
+  if (block_failed(a.dsc)) return;
   constexpr int RT = kHelmThreads / kTile;
   const int n = a.n, s = a.substep, tid = threadIdx.x, nm = a.nmodes, ps = (n | 1) * kTile;
   const int k = tid % kTile, rt = tid / kTile, m = blockIdx.x * kTile + k;

@@ -311,6 +311,13 @@ __device__ __forceinline__ void fixed_bwd(double *x, int n, UF uf) {
   }
 }
 
+// Whether a failed step is to be left untouched, decided once per block: another block of the same grid, or a
+// kernel beside it, may raise the flag while this one starts, and threads that left on their own reading of
+// it would leave the others at barriers that were never set up.
+__device__ __forceinline__ bool block_failed(const DevScalars *dsc) {
+  return __syncthreads_or(threadIdx.x == 0 && dsc->err != 0);
+}
+
 // Row r of an operator spans 2BW+1 columns from here (the near-boundary packing of the first and
 // last BW rows, LABS_full_to_band, module_labs.f90:301-328).
 template <int BW>

@@ -52,7 +52,7 @@ __host__ __device__ constexpr int64_t mean_line_doubles(int bw, int n) {
 template <int BW, bool SM>
 __global__ void __launch_bounds__(256) k_mean(MeanArgs a) {
   extern __shared__ double mean_smem[];
-  if (a.dsc->err) return;
+  if (block_failed(a.dsc)) return;
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, line = warp % 4;
   const bool mine = line < 2 + a.nsc;
   const int n = a.ny, s = a.substep;

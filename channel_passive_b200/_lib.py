@@ -30,6 +30,7 @@ KMM_STAT_NLINES = 58
 KMM_STAT_NSPEC = 18
 KMM_NKERNEL = 8
 KERNEL_NAMES = ("begin_substep", "zinv", "xphys", "update_dt", "zfwd", "hvhg", "helmholtz", "assemble")
+KMM_SOLVER_AUTO, KMM_SOLVER_SWEEPS, KMM_SOLVER_LINES = 0, 1, 2
 KMM_GRID_SINE = 0
 KMM_GRID_TANH = 1
 
@@ -106,6 +107,8 @@ SIGNATURES = {
     "kmm_config_default": (C.c_int, [C.POINTER(KmmConfig)]),
     "kmm_read_input_file": (C.c_int, [C.c_char_p, C.POINTER(KmmConfig)]),
     "kmm_create": (C.c_int, [C.POINTER(KmmConfig), C.POINTER(_P)]),
+    "kmm_create_with_solver": (C.c_int, [C.POINTER(KmmConfig), C.c_int, C.POINTER(_P)]),
+    "kmm_get_solver": (C.c_int, [_P]),
     "kmm_destroy": (C.c_int, [_P]),
     "kmm_get_info": (C.c_int, [_P, C.POINTER(KmmInfo)]),
     "kmm_get_operators": (C.c_int, [_P, _D, _D, _D, _D, _D, _D]),

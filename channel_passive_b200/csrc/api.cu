@@ -456,8 +456,12 @@ int kmm_read_input_file(const char *path, kmm_config *cfg) {
 }
 
 int kmm_create(const kmm_config *cfg, kmm_handle **out) {
-  if (!cfg || !out) {
-    set_error("null argument");
+  return kmm_create_with_solver(cfg, KMM_SOLVER_AUTO, out);
+}
+
+int kmm_create_with_solver(const kmm_config *cfg, int solver, kmm_handle **out) {
+  if (!cfg || !out || solver < KMM_SOLVER_AUTO || solver > KMM_SOLVER_LINES) {
+    set_error(cfg && out ? "unknown solver" : "null argument");
     return KMM_ERR_ARG;
   }
   *out = nullptr;
@@ -554,7 +558,12 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   if ((rc = dalloc(*h, &h->vwall, 2 * (size_t)h->nmodes))) return fail(rc);
   if ((rc = dalloc(*h, &h->zc, (8 + 2 * x2) * (size_t)h->ns))) return fail(rc);
   if ((rc = dalloc(*h, &h->ec, (9 + 2 * x2) * (size_t)h->ns))) return fail(rc);
-  h->lines = line_solver_fits(*h);
+  const bool fits = line_solver_fits(*h);
+  if (solver == KMM_SOLVER_LINES && !fits) {
+    set_error("the line solver's lines do not fit a block's shared memory on this grid");
+    return fail(KMM_ERR_CONFIG);
+  }
+  h->lines = fits && (solver == KMM_SOLVER_LINES || (solver == KMM_SOLVER_AUTO && line_solver_pays(*h)));
   // (the pressure solve keeps its U factors in the first role's region of ub)
   if ((rc = dalloc(*h, &h->ub, (h->lines ? 1 : 3 + x2) * (size_t)split_ub_role(*h)))) return fail(rc);
   if ((rc = dalloc(*h, &h->dvw, 3 * (size_t)h->nmodes))) return fail(rc);
@@ -635,6 +644,11 @@ int kmm_create(const kmm_config *cfg, kmm_handle **out) {
   if (cfg->autotune && (rc = autotune(*h, nullptr))) return fail(rc);
   *out = reinterpret_cast<kmm_handle *>(h);
   return KMM_OK;
+}
+
+int kmm_get_solver(const kmm_handle *hh) {
+  if (!hh) return 0;
+  return reinterpret_cast<const Handle *>(hh)->lines ? KMM_SOLVER_LINES : KMM_SOLVER_SWEEPS;
 }
 
 int kmm_destroy(kmm_handle *hh) {

@@ -142,7 +142,7 @@ struct Handle {
   // The line solver's factors instead of hf, hinf, hdvh, vf (lines.cuh TileFac, tile_factor_doubles each):
   // of theta's operator, the one g and phi share and a second scalar's, made every substep, or with
   // the factor cache per substep and dt; and of v's.
-  bool lines = false;                      // the Helmholtz solves run in line_solver.cu (line_solver_fits)
+  bool lines = false;                      // the per-mode solves run in line_solver.cu
   double *lf = nullptr, *lvf = nullptr;
   unsigned *fcount = nullptr;              // [substep] blocks of k_line_factor done (between launches 0)
   int smem_optin = 0, smem_sm = 0;         // the device's shared memory: most of a block, of an SM
@@ -306,11 +306,12 @@ cudaError_t launch_statistics(Handle &h, cudaStream_t st);
 // whole (L then U), and the kernel that fills it once per handle.
 int64_t vop_lband_doubles(const Handle &h);
 int64_t vop_factor_doubles(const Handle &h);
-// The line solver (line_solver.cu): whether it takes h's grid (called once, by kmm_create, which also
-// learns the device's shared memory from it), doubles of one operator's LU of every mode in its layout,
+// The line solver (line_solver.cu): whether its lines fit h's grid (called once, by kmm_create, which also
+// learns the device's shared memory from it), whether it is the faster solver there, doubles of one operator's LU of every mode in its layout,
 // its set-up (shared-memory limits, v's factors), the factors of a substep (they need its dt alone) and
 // the Helmholtz part of a substep.
 bool line_solver_fits(Handle &h);
+bool line_solver_pays(const Handle &h);
 int64_t tile_factor_doubles(const Handle &h);
 cudaError_t prepare_line_solver(Handle &h, cudaStream_t st);
 cudaError_t launch_line_hvhg(Handle &h, int substep, cudaStream_t st);

@@ -834,7 +834,6 @@ constexpr int64_t kMaxLineModes = 12000;
 bool line_solver_fits(Handle &h) {
   h.smem_optin = smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin);
   h.smem_sm = smem_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor);
-  if (h.nmodes > kMaxLineModes) return false;
   size_t bytes = (size_t)-1;
   with_bw(h.bw, [&]<int BW>() {
     bytes = h.nsc == 2 ? HelmSmem<BW, 2>::bytes(h.ny, 2) : HelmSmem<BW, 1>::bytes(h.ny, 2);
@@ -842,6 +841,8 @@ bool line_solver_fits(Handle &h) {
   });
   return bytes <= (size_t)h.smem_optin;
 }
+
+bool line_solver_pays(const Handle &h) { return h.nmodes <= kMaxLineModes; }
 
 int64_t tile_factor_doubles(const Handle &h) {
   const int64_t tiles = (h.nmodes + kTile - 1) / kTile, bw = h.bw;

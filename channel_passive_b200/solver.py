@@ -120,9 +120,14 @@ def _as_state(U: np.ndarray, cfg: Config, what="U") -> np.ndarray:
 
 
 class Channel:
-    """One channel resident in HBM on one GPU (the GPU half of the drop-in boundary)."""
+    """One channel resident in HBM on one GPU (the GPU half of the drop-in boundary).
 
-    def __init__(self, config: Config | None = None, **overrides):
+    ``solver`` picks the form of the per-mode solves: "auto" (the faster one for the grid), "sweeps" or
+    "lines" (kmm_create_with_solver)."""
+
+    SOLVERS = ("auto", "sweeps", "lines")
+
+    def __init__(self, config: Config | None = None, *, solver: str = "auto", **overrides):
         cfg = config or Config()
         for k, v in overrides.items():
             setattr(cfg, k, v)
@@ -130,7 +135,7 @@ class Channel:
         self._lib = _lib.load()
         h = C.c_void_p()
         c = cfg.to_c()
-        check(self._lib.kmm_create(C.byref(c), C.byref(h)))
+        check(self._lib.kmm_create_with_solver(C.byref(c), self.SOLVERS.index(solver), C.byref(h)))
         self._h = h
         info = KmmInfo()
         check(self._lib.kmm_get_info(self._h, C.byref(info)))
@@ -145,6 +150,11 @@ class Channel:
                                           _dptr(self.D1), _dptr(self.D2), _dptr(self.D0_lu)))
         # (ny, ld) C order = Fortran (ld, ny): present as [r, j] like the reference's A(r, j)
         self.D0, self.D1, self.D2, self.D0_lu = (a.T.copy() for a in (self.D0, self.D1, self.D2, self.D0_lu))
+
+    @property
+    def solver(self) -> str:
+        """The solver in use: "sweeps" or "lines"."""
+        return self.SOLVERS[self._lib.kmm_get_solver(self._h)]
 
     # -- lifetime ---------------------------------------------------------------------
     def close(self):

@@ -153,6 +153,16 @@ int kmm_read_input_file(const char *path, kmm_config *cfg);
  * module_runge_kutta.f90:28-54, module_ppdfftw.f90:499-588): builds the B-spline
  * operators, allocates the HBM-resident state and plans the transforms. */
 int kmm_create(const kmm_config *cfg, kmm_handle **out);
+/* The per-mode solves of a step (hvhg, solve_t, solve_g, solve_v_f, solve_u_w) have two forms with the
+ * same results to rounding: sweeps that stream every line through global memory, and a line solver that
+ * holds a tile of modes in shared memory.  kmm_create picks the faster one for the grid;
+ * kmm_create_with_solver takes the caller's choice (KMM_ERR_CONFIG for a line solver whose lines do not
+ * fit a block's shared memory), and kmm_get_solver reports the one in use (0 for a null handle). */
+#define KMM_SOLVER_AUTO 0
+#define KMM_SOLVER_SWEEPS 1
+#define KMM_SOLVER_LINES 2
+int kmm_create_with_solver(const kmm_config *cfg, int solver, kmm_handle **out);
+int kmm_get_solver(const kmm_handle *h);
 int kmm_destroy(kmm_handle *h);
 int kmm_get_info(const kmm_handle *h, kmm_info *info);
 

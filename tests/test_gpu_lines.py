@@ -1,15 +1,20 @@
-"""The line solver of the per-mode solves (line_solver.cu) and the mean lines (k_mean) at the sizes where
-they can go wrong, against the numpy oracle: the smallest ny that a spline order takes (the first and last
-rows' wide profiles overlap), the edges of the staged chunks (ny = bw + 24 c and one more), even ny, mode
-counts that are no multiple of a tile, every band width in use, one and two scalars, control, both time
-step rules and both precisions.  Tolerances: FP64 1e-11 of the field as the other trajectory tests,
-mixed 1e-5."""
+"""Both forms of the per-mode solves, the line solver (line_solver.cu) and the sweeps
+(wavespace_split.cu), and the mean lines (k_mean), against the numpy oracle at the sizes where they can go
+wrong: the smallest ny that a spline order takes (the first and last rows' wide profiles overlap), the
+edges of the staged chunks (ny = bw + 24 c and one more), even ny, mode counts that are no multiple of a
+tile, every band width (2 to 7), one and two scalars, control, both time step rules and both precisions;
+and tall grids: one block of the line solver an SM (ny of 140 and more at band width 4), its last ny (367)
+and the sweeps that take over, the mean lines in global memory (ny of 568 and more).  Tolerances: FP64
+1e-11 of the field as the other trajectory tests, mixed 1e-5; above ny = 129, the tallest of those tests,
+1e-11 times (ny / 129)^2, as the rounding of the second derivatives goes with the inverse square of the
+spacing."""
 import ctypes
 
 import numpy as np
 import pytest
 
-from channel_passive_b200 import Channel
+from channel_passive_b200 import Channel, KmmError
+from channel_passive_b200 import _lib
 from oracle import kmm as okmm
 from tests.helpers import STATE_SLOTS, STATE_SLOTS2, make_pair, oracle_ctrl, rel_l2, seeded_state, with_scalar2
 
@@ -17,10 +22,11 @@ pytestmark = pytest.mark.gpu
 
 SIZES = [  # labs_k, ny
     (6, 18), (6, 19), (6, 28), (6, 29), (6, 52), (6, 77), (4, 10), (4, 26), (4, 51), (5, 14), (5, 40), (7, 18),
-    (7, 30), (8, 22), (8, 33), (10, 26), (10, 45)]
+    (7, 30), (8, 22), (8, 33), (10, 26), (10, 45), (11, 31), (11, 32), (12, 55)]
+SOLVERS = ["lines", "sweeps"]
 
 
-def _compare(cfg, p, nsteps, tol, scalars=1):
+def _compare(cfg, p, nsteps, tol, scalars=1, solver="auto", expect=None):
     ops = okmm.make_operators(p)
     U = seeded_state(cfg, ops.y)
     if scalars == 2:
@@ -29,7 +35,8 @@ def _compare(cfg, p, nsteps, tol, scalars=1):
     Uo, RKo, dt = U.copy(), RK.copy(), 0.01
     for _ in range(nsteps):
         dt, sc = okmm.rk3_step(Uo, RKo, ops, p, dt, ctrl=oracle_ctrl(ops, p))
-    with Channel(cfg) as ch:
+    with Channel(cfg, solver=solver) as ch:
+        assert ch.solver == (expect or solver)
         ch.set_initial_data_uvw(U, 0.01)
         out = ch.step(nsteps)
         Ug, RKg = ch.download_state(U.shape[0])
@@ -40,18 +47,37 @@ def _compare(cfg, p, nsteps, tol, scalars=1):
     assert abs(out["wall_shear_stress"] - sc.wall_shear_stress) <= 10 * tol * abs(sc.wall_shear_stress)
 
 
+@pytest.mark.parametrize("solver", SOLVERS)
 @pytest.mark.parametrize("labs_k,ny", SIZES)
-def test_lines_match_oracle(labs_k, ny):
+def test_lines_match_oracle(labs_k, ny, solver):
     cfg, p = make_pair(nx=12, ny=ny, nz=18, control_amp=-0.7, fixed_dt=ny % 2, labs_k=labs_k)
     p.labs_k = labs_k
-    _compare(cfg, p, 2, 1e-11)
+    _compare(cfg, p, 2, 1e-11, solver=solver)
 
 
+@pytest.mark.parametrize("solver", SOLVERS)
 @pytest.mark.parametrize("ny", [33, 53])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_two_scalars_match_oracle(ny, precision):
+def test_two_scalars_match_oracle(ny, precision, solver):
     cfg, p = make_pair(nx=16, ny=ny, nz=16, control_amp=-0.7, fixed_dt=0, precision=precision, n_scalar=2)
-    _compare(cfg, p, 2, 1e-5 if precision else 1e-11, scalars=2)
+    _compare(cfg, p, 2, 1e-5 if precision else 1e-11, scalars=2, solver=solver)
+
+
+@pytest.mark.parametrize("ny,scalars,expect", [
+    (139, 1, "lines"), (140, 1, "lines"), (193, 1, "lines"), (367, 1, "lines"), (368, 1, "sweeps"),
+    (568, 1, "sweeps"), (80, 2, "lines"), (141, 2, "lines"), (261, 2, "lines"), (262, 2, "sweeps"), (426, 2, "sweeps")])
+def test_tall_grids_match_oracle(ny, scalars, expect):
+    cfg, p = make_pair(nx=8, ny=ny, nz=10, control_amp=-0.7, fixed_dt=ny % 2, n_scalar=scalars)
+    _compare(cfg, p, 1, 1e-11 * max(1.0, ny / 129) ** 2, scalars=scalars, expect=expect)
+
+
+def test_the_caller_can_choose_the_solver():
+    cfg, p = make_pair(nx=16, ny=368, nz=16)
+    with Channel(cfg, solver="sweeps") as ch:
+        assert ch.solver == "sweeps"
+    with pytest.raises(KmmError) as e:
+        Channel(cfg, solver="lines")
+    assert e.value.code == _lib.KMM_ERR_CONFIG
 
 
 def test_kept_factors_carry_their_own_time_step():

@@ -161,9 +161,10 @@ def _wavespace_inputs(cfg, rng):
     return U, RK
 
 
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
 @pytest.mark.parametrize("substep", [1, 2, 3])
 @pytest.mark.parametrize("control", [0.0, -1.0])
-def test_wavespace_matches_oracle(substep, control):
+def test_wavespace_matches_oracle(substep, control, solver):
     cfg, p, ops = _setup(nx=16, ny=33, nz=16, control_amp=control)
     rng = np.random.default_rng(100 + substep)
     U, RK = _wavespace_inputs(cfg, rng)
@@ -171,7 +172,7 @@ def test_wavespace_matches_oracle(substep, control):
     Uo, RKo = U.copy(), RK.copy()
     sc = okmm.Scalars()
     okmm.wavespace(Uo, RKo, ops, p, substep, dt, sc, oracle_ctrl(ops, p))
-    with Channel(cfg) as ch:
+    with Channel(cfg, solver=solver) as ch:
         Ud, RKd = _cplx(U), _cplx(RK)
         out = ch.wavespace(Ud, RKd, substep, dt)
         Ug, RKg = Ud.cpu().numpy(), RKd.cpu().numpy()
@@ -186,7 +187,7 @@ def test_wavespace_matches_oracle(substep, control):
         assert abs(out["wall_theta_stress"] - sc.wall_theta_stress) <= 1e-12 * abs(sc.wall_theta_stress)
 
 
-def _run_pair(cfg, p, ops, nsteps, dt=0.01, use_graph=True, ctrl=True):
+def _run_pair(cfg, p, ops, nsteps, dt=0.01, use_graph=True, ctrl=True, solver="auto"):
     U = seeded_state(cfg, ops.y)
     RK = okmm.set_initial_data_uvw(U.copy(), ops, p)
     Uo, RKo = U.copy(), RK.copy()
@@ -196,7 +197,7 @@ def _run_pair(cfg, p, ops, nsteps, dt=0.01, use_graph=True, ctrl=True):
     d = dt
     for _ in range(nsteps):
         d, sco = okmm.rk3_step(Uo, RKo, ops, p, d, sco, dyr, c)
-    with Channel(cfg) as ch:
+    with Channel(cfg, solver=solver) as ch:
         ch.set_initial_data_uvw(U, dt)
         if use_graph:
             out = ch.step(nsteps)
@@ -218,19 +219,21 @@ def test_set_initial_data_uvw_matches_oracle():
     assert rel_l2(RKg, RKo) < 1e-13
 
 
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
 @pytest.mark.parametrize("control", [0.0, -1.0])
-def test_substeps_match_oracle(control):
+def test_substeps_match_oracle(control, solver):
     cfg, p, ops = _setup(nx=16, ny=33, nz=16, control_amp=control)
-    Ug, RKg, out, Uo, RKo, sco = _run_pair(cfg, p, ops, 2, use_graph=False)
+    Ug, RKg, out, Uo, RKo, sco = _run_pair(cfg, p, ops, 2, use_graph=False, solver=solver)
     for s in STATE_SLOTS:
         assert rel_l2(Ug[s], Uo[s]) < 1e-12, s
     assert rel_l2(RKg, RKo) < 1e-12
     assert abs(out["velmax"] - sco.velmax) <= 1e-12 * sco.velmax
 
 
-def test_graph_step_matches_oracle_cfl_dt():
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
+def test_graph_step_matches_oracle_cfl_dt(solver):
     cfg, p, ops = _setup(nx=16, ny=33, nz=24, fixed_dt=0, control_amp=-1.0)
-    Ug, RKg, out, Uo, RKo, sco = _run_pair(cfg, p, ops, 4, dt=0.0, use_graph=True)
+    Ug, RKg, out, Uo, RKo, sco = _run_pair(cfg, p, ops, 4, dt=0.0, use_graph=True, solver=solver)
     for s in STATE_SLOTS:
         assert rel_l2(Ug[s], Uo[s]) < 1e-11, s
     assert abs(out["dt"] - sco.dt) <= 1e-13 * sco.dt

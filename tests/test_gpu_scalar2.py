@@ -20,16 +20,17 @@ from tests.helpers import STATE_SLOTS, STATE_SLOTS2, make_pair, oracle_ctrl, rel
 pytestmark = pytest.mark.gpu
 
 
-def test_second_scalar_with_the_first_ones_parameters_reproduces_it():
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
+def test_second_scalar_with_the_first_ones_parameters_reproduces_it(solver):
     kw = dict(nx=16, ny=33, nz=16, control_amp=-1.0, fixed_dt=1, precision=0)
     cfg1, p = make_pair(**kw)
     cfg2, _ = make_pair(n_scalar=2, pr2=cfg1.pr, bulk_t2=cfg1.bulk_t, **kw)
     U = seeded_state(cfg1, okmm.make_operators(p).y)
-    with Channel(cfg1) as ch:
+    with Channel(cfg1, solver=solver) as ch:
         ch.set_initial_data_uvw(U, 0.01)
         s1 = ch.step(3)
         U1, _ = ch.download_state(10)
-    with Channel(cfg2) as ch:
+    with Channel(cfg2, solver=solver) as ch:
         ch.set_initial_data_uvw(with_scalar2(U), 0.01)
         s2 = ch.step(3)
         U2, RK2 = ch.download_state(11)
@@ -43,8 +44,9 @@ def test_second_scalar_with_the_first_ones_parameters_reproduces_it():
     assert s2["phi_dpdx"] == s1["phi_dpdx"] and s2["phi_dtdx"] == s1["phi_dtdx"]
 
 
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
 @pytest.mark.parametrize("precision,tol,nsteps", [(0, 1e-11, 3), (1, 1e-5, 20)])
-def test_second_scalar_matches_oracle(precision, tol, nsteps):
+def test_second_scalar_matches_oracle(precision, tol, nsteps, solver):
     cfg, p = make_pair(nx=32, ny=33, nz=32, control_amp=-1.0, fixed_dt=1, precision=precision, n_scalar=2,
                        pr2=0.2, bulk_t2=0.5)
     ops = okmm.make_operators(p)
@@ -58,7 +60,7 @@ def test_second_scalar_matches_oracle(precision, tol, nsteps):
     ctrl = oracle_ctrl(ops, p)
     for _ in range(nsteps):
         _, sco = okmm.rk3_step(Uo, RKo, ops, p, 0.01, ctrl=ctrl)
-    with Channel(cfg) as ch:
+    with Channel(cfg, solver=solver) as ch:
         ch.set_initial_data_uvw(U, 0.01)
         scg = ch.step(nsteps)
         Ug, RKg = ch.download_state(11)
@@ -94,7 +96,7 @@ def test_second_scalar_block_shapes_are_bit_identical(precision):
                   dict(helm_modes_per_block=64, helm_tables_shared=1),
                   dict(helm_modes_per_block=96, helm_tables_shared=1),
                   dict(helm_modes_per_block=96, helm_tables_shared=0)):
-        with Channel(cfg) as ch:
+        with Channel(cfg, solver="sweeps") as ch:
             ch.set_tuning(**shape)
             assert ch.tuning["helm_modes_per_block"] == shape["helm_modes_per_block"]
             ch.set_initial_data_uvw(U, 0.01)

@@ -12,8 +12,8 @@ from tests.helpers import STATE_SLOTS, make_pair, seeded_state
 pytestmark = pytest.mark.gpu
 
 
-def _run(cfg, U, tuning=None, nsteps=2):
-    with Channel(cfg) as ch:
+def _run(cfg, U, tuning=None, nsteps=2, solver="auto"):
+    with Channel(cfg, solver=solver) as ch:
         if tuning:
             ch.set_tuning(**tuning)
         ch.set_initial_data_uvw(U, 0.01)
@@ -21,12 +21,14 @@ def _run(cfg, U, tuning=None, nsteps=2):
         return ch.download_state(10)[0]
 
 
+# the solver's shapes are the sweeps'; the line solver, which these grids get by default, has one
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_every_candidate_shape_is_bit_identical(precision):
+def test_every_candidate_shape_is_bit_identical(precision, solver):
     cfg, p = make_pair(nx=64, ny=65, nz=64, control_amp=-1.0, precision=precision)
     U = seeded_state(cfg, okmm.make_operators(p).y)
-    ref = _run(cfg, U)
-    with Channel(cfg) as ch:
+    ref = _run(cfg, U, solver=solver)
+    with Channel(cfg, solver=solver) as ch:
         rep = ch.autotune()
     assert rep["tuned"] == 1
     # the candidates: variant shapes reported by the tuner's timings are tried one knob at a time
@@ -44,16 +46,17 @@ def test_every_candidate_shape_is_bit_identical(precision):
     cases += [dict(helm_modes_per_block=mb, helm_tables_shared=ts, helm_stage_ahead=sa)
               for mb in (32, 64, 128) for ts in (0, 1) for sa in (1, 2)]
     for case in cases:
-        got = _run(cfg, U, case)
+        got = _run(cfg, U, case, solver=solver)
         for f in STATE_SLOTS:
             assert np.array_equal(got[f], ref[f]), (case, f)
 
 
-def test_autotune_keeps_the_state_and_reports_its_choice():
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
+def test_autotune_keeps_the_state_and_reports_its_choice(solver):
     cfg, p = make_pair(nx=64, ny=65, nz=64, control_amp=-1.0, precision=1)
     U = seeded_state(cfg, okmm.make_operators(p).y)
-    ref = _run(cfg, U, nsteps=3)
-    with Channel(cfg) as ch:
+    ref = _run(cfg, U, nsteps=3, solver=solver)
+    with Channel(cfg, solver=solver) as ch:
         ch.set_initial_data_uvw(U, 0.01)
         ch.step(1)
         before, rk_before = ch.download_state(10)
@@ -93,8 +96,9 @@ def test_create_with_autotune_flag():
     assert t["u_layout"] in (0, int(np.argmin(t["ms_layout"])))
 
 
+@pytest.mark.parametrize("solver", ["auto", "sweeps"])
 @pytest.mark.parametrize("precision", [0, 1])
-def test_factor_cache_gives_the_same_numbers_across_dt_changes(precision):
+def test_factor_cache_gives_the_same_numbers_across_dt_changes(precision, solver):
     """factor_cache (fixed time step, the default there): the Helmholtz sweeps that read each
     substep's cached operator factors and influence solutions give the per-substep factorisation's
     results bit for bit, also when dt changes between steps (the cache is rebuilt for the new dt)
@@ -103,7 +107,7 @@ def test_factor_cache_gives_the_same_numbers_across_dt_changes(precision):
     U = seeded_state(cfg, okmm.make_operators(p).y)
     out = {}
     for fc in (0, 1):
-        with Channel(cfg) as ch:
+        with Channel(cfg, solver=solver) as ch:
             assert ch.tuning["factor_cache"] == 1
             ch.set_tuning(factor_cache=fc)
             assert ch.tuning["factor_cache"] == fc

@@ -675,6 +675,15 @@ __global__ void __launch_bounds__(kHelmThreads, 3) k_line_hvhg(HvhgArgs a) {
   }
 }
 
+// Ring slots of k_lines: three if that many leave room for kHelmBlocks blocks an SM (or for the one that fits).
+template <int BW, int NS>
+int line_stages(const Handle &h) {
+  using L = HelmSmem<BW, NS>;
+  const size_t b2 = L::bytes(h.ny, 2), b3 = L::bytes(h.ny, 3);
+  return b3 <= (size_t)h.smem_optin && (kHelmBlocks * (b3 + 1024) <= (size_t)h.smem_sm ||
+                                        kHelmBlocks * (b2 + 1024) > (size_t)h.smem_sm) ? 3 : 2;
+}
+
 // Shared memory of k_line_hvhg: its planes, and at least the probes' sums.
 size_t line_hvhg_bytes(const Handle &h) {
   const size_t planes = (size_t)(h.nsc == 2 ? 10 : 8) * (size_t)(h.ny | 1) * kTile;
@@ -731,16 +740,9 @@ cudaError_t helm_bw(Handle &h, int substep, const double *dt_ptr, cudaStream_t s
   const HelmArgs a = helm_args(h, substep, dt_ptr);
   const unsigned tiles = (unsigned)((h.nmodes + kTile - 1) / kTile);
   auto go = [&]<typename PT, int NS>() {
-    using L = HelmSmem<BW, NS>;
-    // three ring slots if that many leave room for kHelmBlocks blocks an SM (or for the one that fits)
-    int stages = 2;
-    if (L::bytes(h.ny, 3) <= (size_t)h.smem_optin &&
-        (kHelmBlocks * (L::bytes(h.ny, 3) + 1024) <= (size_t)h.smem_sm ||
-         kHelmBlocks * (L::bytes(h.ny, 2) + 1024) > (size_t)h.smem_sm))
-      stages = 3;
     HelmArgs b = a;
-    b.stages = stages;
-    k_lines<BW, PT, NS><<<tiles, kHelmThreads, L::bytes(h.ny, stages), st>>>(b);
+    b.stages = line_stages<BW, NS>(h);
+    k_lines<BW, PT, NS><<<tiles, kHelmThreads, HelmSmem<BW, NS>::bytes(h.ny, b.stages), st>>>(b);
   };
   if (h.mixed) h.nsc == 2 ? go.template operator()<float2, 2>() : go.template operator()<float2, 1>();
   else h.nsc == 2 ? go.template operator()<double2, 2>() : go.template operator()<double2, 1>();
@@ -822,14 +824,60 @@ template <typename F> auto with_bw(int bw, F &&f) {
   }
 }
 
-}  // namespace
+// Whether two blocks of k_lines are resident on an SM.
+bool two_lines(const Handle &h) {
+  bool two = false;
+  with_bw(h.bw, [&]<int BW>() {
+    const size_t bytes = h.nsc == 2 ? HelmSmem<BW, 2>::bytes(h.ny, line_stages<BW, 2>(h))
+                                    : HelmSmem<BW, 1>::bytes(h.ny, line_stages<BW, 1>(h));
+    two = kHelmBlocks * (bytes + 1024) <= (size_t)h.smem_sm;
+    return cudaSuccess;
+  });
+  return two;
+}
 
-// Up to here the line solver is the faster one: on 64x65x64 the Helmholtz part of a substep takes 41 us
-// against 157 with the sweeps of wavespace_split.cu, on 128x97x128 (8192 modes) 177 against 266, on
-// 144x97x144 (10368) 208 against 288, with two scalars on 128x97x128 373 against 415; from about 160x160
-// (12800 modes) the sweeps have enough warps to reach two thirds of the memory rate: 503 against 499 on
-// 160x129x160, 459 against 422 on 192x129x192.
-constexpr int64_t kMaxLineModes = 12000;
+// Up to how many modes the line solver is the faster one, from whole steps with either solver (ratio line
+// solver / sweeps, FP64 and mixed, ny from 33 to 353, 4096 to 15360 modes; below 4096 it is 0.25 to 0.9
+// everywhere).  With more modes the sweeps have the warps to hide their latency; the line solver loses
+// residency with ny, k_line_hvhg's second block an SM above all (its planes: ny = 227 with one scalar, 181
+// with two), and so does its lead.  Sweeps that have to factor each substep (a CFL time step, two
+// scalars) lose more the wider the band.
+int64_t line_modes(const Handle &h) {
+  const int bw = h.bw;
+  const bool cached = factor_cache_possible(h);
+  const bool two_hvhg = 2 * (line_hvhg_bytes(h) + 1024) <= (size_t)h.smem_sm;
+  constexpr int64_t all = 12000;  // (12800 modes at band width 4: 0.95 to 1.07)
+  if (!cached && bw >= 6) return all;  // 0.43 to 1.00 up to 13824 modes, also with one block an SM
+  if (!two_hvhg) {
+    if (cached) return bw <= 4 ? 8700   // 8192 modes 0.92 to 0.98, 9216 0.97 to 1.05
+                       : 7000;          // 6144 modes 0.91 to 0.98, 8192 1.00 to 1.08
+    if (h.nsc == 2) return bw == 4 ? 6000   // 5120 modes 0.90 to 0.95, 6144 0.99 to 1.04
+                           : 7000;          // 6144 modes 0.94 to 0.98, 8192 1.03 to 1.06
+    return bw <= 4 ? 7000   // 6144 modes 0.92 to 0.97, 8192 1.01 to 1.04
+           : 8700;          // 8192 modes 0.93, 9216 1.00
+  }
+  if (cached) {
+    if (bw <= 4) return h.ny < 48 ? 10900 : all;  // 11520 modes 0.92 to 0.98, at ny = 33 0.99 to 1.03
+    if (h.ny < 48) return 7000;                   // 6144 modes 0.88, 8192 1.03 to 1.05
+    return bw == 5 ? 10900   // 10368 modes 0.92 to 1.01, 11520 0.98 to 1.05
+           : 9000;           // 8192 modes 0.93 to 1.03, 9216 0.97 to 1.07
+  }
+  if (h.nsc == 2) {
+    // 11520 modes 0.95 to 1.00 (ny = 33: 10240 0.98 to 1.02); with one block of k_lines an SM 6144 modes 0.86
+    // to 0.93 and 8192 0.98 to 1.03, at band width 5 11520 modes 0.97 to 1.02
+    if (bw == 5) return all;
+    if (!two_lines(h)) return 7600;
+    return h.ny < 48 ? 10000 : all;
+  }
+  if (bw <= 3) {
+    if (h.ny < 48) return 7000;          // 6144 modes 0.86 to 0.95, 8192 1.03 to 1.06
+    if (!two_lines(h)) return 8700;      // 8192 modes 0.96 to 1.03, 9216 0.99 to 1.05
+    return h.ny < 96 ? 11000 : all;      // at ny = 65 10368 modes 0.99 to 1.01, 11520 1.02 to 1.04
+  }
+  return h.ny < 48 && bw == 4 ? 10900 : all;  // 11520 modes 0.95 to 1.02, at ny = 33 1.01 to 1.02
+}
+
+}  // namespace
 
 bool line_solver_fits(Handle &h) {
   h.smem_optin = smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin);
@@ -842,7 +890,7 @@ bool line_solver_fits(Handle &h) {
   return bytes <= (size_t)h.smem_optin;
 }
 
-bool line_solver_pays(const Handle &h) { return h.nmodes <= kMaxLineModes; }
+bool line_solver_pays(const Handle &h) { return h.nmodes <= line_modes(h); }
 
 int64_t tile_factor_doubles(const Handle &h) {
   const int64_t tiles = (h.nmodes + kTile - 1) / kTile, bw = h.bw;

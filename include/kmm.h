@@ -95,8 +95,9 @@ typedef struct kmm_info {
 
 /* Launch shapes chosen by kmm_autotune (the hand-tuned defaults before it runs), and the
  * measured device time (ms) of every candidate it tried. */
-/* On grids of up to 12000 modes the Helmholtz solves run in the line solver, which has one shape:
- * u_layout, assemble_threads and the helm_* fields are checked and reported there and change nothing. */
+/* The per-mode solves' fields are those of the sweeps.  A handle with the line solver (kmm_get_solver), which
+ * has one shape, checks and reports modes_per_block, tables_shared, hvhg_stage_ahead, u_layout,
+ * assemble_threads and the helm_* fields, and they change nothing. */
 typedef struct kmm_tuning {
   int32_t z_lines_per_block;  /* z transforms (y_to_x, x_to_y): kx lines a block transforms */
   int32_t x_rows_per_block;   /* x pass (dft_x_realspace): z rows a block takes */
@@ -280,8 +281,8 @@ int kmm_set_tuning(kmm_handle *h, const kmm_tuning *t);
 #define KMM_K_ZFWD 4        /* x_to_y: z forward transform of the 8 products (+ rescale) */
 #define KMM_K_HVHG 5        /* wavespace part 1: control probe, mean-mode fork, hvhg D0 solves */
 #define KMM_K_HELMHOLTZ 6   /* wavespace part 2: theta, g, phi and v Helmholtz solves */
-#define KMM_K_ASSEMBLE 7    /* wavespace part 3: C1/C2 assembly, u and w (up to 12000 modes part of
-                               KMM_K_HELMHOLTZ, and nothing here; the join of the mean-mode
+#define KMM_K_ASSEMBLE 7    /* wavespace part 3: C1/C2 assembly, u and w (with the line solver part
+                               of KMM_K_HELMHOLTZ, and nothing here; the join of the mean-mode
                                lines, which run beside the solver kernels, is outside every id) */
 
 /* Runs nsteps RK3 steps launching kernel by kernel with a CUDA event pair around every

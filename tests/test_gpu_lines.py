@@ -104,3 +104,16 @@ def test_kept_factors_carry_their_own_time_step():
     for f in STATE_SLOTS:
         assert np.array_equal(out[0][0][f], out[1][0][f]), f
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("nx,ny,nz,kw,expect", [
+    (128, 97, 128, dict(fixed_dt=1), "lines"), (128, 225, 128, dict(fixed_dt=0), "lines"),
+    (128, 257, 128, dict(fixed_dt=0), "sweeps"), (128, 257, 128, dict(fixed_dt=1), "lines"),
+    (144, 257, 144, dict(fixed_dt=1), "sweeps"), (160, 65, 160, dict(fixed_dt=1), "sweeps"),
+    (128, 65, 128, dict(n_scalar=2), "lines"), (128, 129, 128, dict(n_scalar=2), "sweeps"),
+    (128, 33, 128, dict(fixed_dt=1, labs_k=10), "sweeps"), (128, 193, 128, dict(fixed_dt=0, labs_k=10), "lines")])
+def test_the_faster_solver_is_the_default(nx, ny, nz, kw, expect):
+    """One grid on each side of the rule's lines (line_modes); the figures stand there."""
+    cfg, _ = make_pair(nx=nx, ny=ny, nz=nz, **kw)
+    with Channel(cfg) as ch:
+        assert ch.solver == expect

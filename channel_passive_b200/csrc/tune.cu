@@ -13,6 +13,9 @@
 //                  or two rows of staging look-ahead, where a block's shared memory holds the
 //                  shape; then the U factor storage layout,
 //   assembly       threads per block.
+// Where the candidates of a group are one and the same launch (the solver's on a line-solver handle, the
+// transforms' off the tuned lengths) it is timed once, each candidate reports that time, and the entry
+// shapes stay.
 // Each candidate runs once to warm up, then kReps times between CUDA events on the handle's
 // stream; the minimum of the means wins.  Last, whole steps through the step graph decide which
 // of those picks stay, one knob group at a time from the shapes the handle had before: in the
@@ -110,6 +113,7 @@ int autotune(Handle &h, kmm_tuning *out) {
   // (where the grid allows the tile map)
   double best_z = 0.0;
   int bz = 0, bt = 0;
+  const bool one_z = !fft4_supported(h.nz32), one_x = !fft4_supported(h.nx32);
   for (int t = 0; t < 2; ++t)
     for (int v = 0; v < 3; ++v) {
       if (t && !z_tma_possible(h, v)) continue;
@@ -121,15 +125,16 @@ int autotune(Handle &h, kmm_tuning *out) {
         return e;
       };
       double *slot = t ? &rep.ms_z_tma[v] : &rep.ms_z[v];
-      if ((rc = measure(none, body, slot))) return rc;
+      if (one_z && best_z > 0.0) *slot = best_z;
+      else if ((rc = measure(none, body, slot))) return rc;
       if (best_z == 0.0 || *slot < best_z) {
         best_z = *slot;
         bz = v;
         bt = t;
       }
     }
-  h.tune.z = bz;
-  h.tune.ztma = bt;
+  h.tune.z = one_z ? entry.z : bz;
+  h.tune.ztma = one_z ? entry.ztma : bt;
   // x pass, each run on fresh z-inverse slabs
   for (int v = 0; v < 3; ++v) {
     h.tune.x = v;
@@ -138,9 +143,10 @@ int autotune(Handle &h, kmm_tuning *out) {
       return KMM_OK;
     };
     auto body = [&]() { return launch_xphys(h, h.MID, 2, st); };
-    if ((rc = measure(prep, body, &rep.ms_x[v]))) return rc;
+    if (one_x && v > 0) rep.ms_x[v] = rep.ms_x[0];
+    else if ((rc = measure(prep, body, &rep.ms_x[v]))) return rc;
   }
-  h.tune.x = best(rep.ms_x, 3);
+  h.tune.x = one_x ? entry.x : best(rep.ms_x, 3);
   // the per-mode solves of substep 2 on products of the saved state
   {
     TUNE_CUDA(launch_zinv(h, h.S, h.MID, nfld, st));
@@ -173,7 +179,8 @@ int autotune(Handle &h, kmm_tuning *out) {
           h.tune.hvstage = sa;
           double ms = 0.0;
           auto body = [&]() { return launch_ws_hvhg(h, 2, nullptr, st); };
-          if ((rc = measure(restore_joined, body, &ms))) return rc;
+          if (h.lines && best_ms > 0.0) ms = best_ms;
+          else if ((rc = measure(restore_joined, body, &ms))) return rc;
           rep.ms_hvhg[((g - 1) * 2 + sh) * 3 + sa] = ms;
           keep_min(rep.ms_modes[g - 1], ms);
           keep_min(rep.ms_tables[sh], ms);
@@ -211,7 +218,8 @@ int autotune(Handle &h, kmm_tuning *out) {
           h.tune.hstab = sh;
           h.tune.stage = sa;
           double ms = 0.0;
-          if ((rc = measure(after_hvhg, helm, &ms))) return rc;
+          if (h.lines && best_ms > 0.0) ms = best_ms;
+          else if ((rc = measure(after_hvhg, helm, &ms))) return rc;
           rep.ms_helm[(gi * 2 + sh) * 2 + sa - 1] = ms;
           if (best_ms == 0.0 || ms < best_ms) {
             best_ms = ms;
@@ -226,7 +234,8 @@ int autotune(Handle &h, kmm_tuning *out) {
     rep.ms_layout[0] = best_ms;
   }
   h.tune.ulayout = 1;
-  if ((rc = measure(after_hvhg, helm, &rep.ms_layout[1]))) return rc;
+  if (h.lines) rep.ms_layout[1] = rep.ms_layout[0];
+  else if ((rc = measure(after_hvhg, helm, &rep.ms_layout[1]))) return rc;
   h.tune.ulayout = rep.ms_layout[1] < rep.ms_layout[0] ? 1 : 0;
   auto solve = [&]() {
     cudaError_t e = launch_ws_hvhg(h, 2, nullptr, st);
@@ -244,9 +253,17 @@ int autotune(Handle &h, kmm_tuning *out) {
       return KMM_OK;
     };
     auto body = [&]() { return launch_ws_assemble(h, 2, nullptr, st); };
-    if ((rc = measure(prep, body, &rep.ms_assemble[i]))) return rc;
+    if (h.lines && i > 0) rep.ms_assemble[i] = rep.ms_assemble[0];
+    else if ((rc = measure(prep, body, &rep.ms_assemble[i]))) return rc;
   }
   h.tune.asm_threads = athreads[best(rep.ms_assemble, 3)];
+  if (h.lines) {
+    const Tuning transforms = h.tune;
+    h.tune = entry;
+    h.tune.z = transforms.z;
+    h.tune.ztma = transforms.ztma;
+    h.tune.x = transforms.x;
+  }
   // Whole steps through the step graph (the solver kernels beside the mean lines on the side
   // stream, as the step runs them) decide which picks stay: starting from the shapes the handle
   // had, each knob group takes its per-kernel pick only where the step gets 1% faster with it.  With

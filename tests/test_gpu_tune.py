@@ -130,3 +130,18 @@ def test_factor_cache_needs_a_fixed_time_step():
         with pytest.raises(KmmError) as e:
             ch.set_tuning(factor_cache=1)
         assert e.value.code == _lib.KMM_ERR_ARG
+
+
+def test_autotune_times_a_single_candidate_once():
+    """A line-solver handle has one solver shape, and a length off the tuned list (135) one transform
+    shape: every candidate reports the one time, and the shapes stay as they were."""
+    cfg, _ = make_pair(nx=90, ny=33, nz=90, precision=1)
+    with Channel(cfg, solver="lines") as ch:
+        before = ch.tuning
+        rep = ch.autotune()
+        after = ch.tuning
+    for name in ("ms_z", "ms_x", "ms_modes", "ms_tables", "ms_hvhg", "ms_layout", "ms_helm", "ms_assemble"):
+        assert len({x for x in rep[name] if x > 0}) == 1, name
+    for name, value in before.items():
+        if not name.startswith("ms_") and name != "tuned":
+            assert after[name] == value, name

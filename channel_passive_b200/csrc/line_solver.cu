@@ -41,7 +41,7 @@ struct HelmArgs {
 // ------------------------------------------------------------------------------------------
 // k_line_factor: one thread per mode and operator; op = blockIdx.y (0 theta, 1 g and phi, 2 theta2), or
 // v's operator with a.fac[0] null.  LuSweep's profile Crout LU, stored by tile.  A no-op while the
-// sets hold this dt (a fixed time step: 3 us against 0.5 ms once a substep and run).
+// sets hold this dt (a fixed time step: 3 us against 112 us on 128x97x128 once a substep and run).
 // The sets and the dt they hold are written here together, by the last block to finish: it runs beside the
 // transforms, and whatever becomes of the substep after it, the mark is that of the sets.  (For the same
 // reason it does not look at the error flag: some blocks would leave and others not.)
@@ -50,46 +50,43 @@ __global__ void __launch_bounds__(32) k_line_factor(HelmArgs a) {
   const bool vop = a.fac[0] == nullptr;
   if (!vop && a.cached && *a.fcdt == *a.dt_ptr) return;
   const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= a.nmodes) return;
   const int n = a.n, op = blockIdx.y;
-  if (m < a.nmodes) {
-    const Tabs<BW> tb = tabs_at<BW>(a.tabs, n);
-    const double k2 = mode_k((int)m, a.nxh, a.nz, a.lmfxr, a.lmfzr).k2;
-    double *f = (vop ? a.vf : a.fac[op]) + (m / kTile) * TileFac<BW>::size(n);
-    const int km = (int)(m % kTile);
-    double ca = 0.0, cb = 0.0;
-    if (!vop) {
-      cb = *a.dt_ptr * rkc(2, a.substep) * (op == 0 ? a.nu / a.pr : op == 1 ? a.nu : a.nu / a.pr2);
-      ca = 1.0 + cb * k2;
-    }
-    LuSweep<BW, 0, 0, true, TileU<BW>> lu;
-    lu.init(n, TileU<BW>{f + TileFac<BW>::bwd(n), f + TileFac<BW>::bx(n) + km, n, km});
-    const double2 bc[1] = {z2(0.0, 0.0)};
-    const double br[1] = {0.0};
-    double2 zc[1];
-    double zr[1];
-    for (int r = 1; r <= n; ++r) {
-      lu.step(r, [&](int rr, double *row, bool c) {
-        if (vop) vrow<BW>(tb, rr, n, k2, row, c);
-        else helm_row<BW>(tb, rr, n, ca, cb, row, c);
-      }, bc, br, zc, zr);
-      const int q = r - 1;  // 0-based
-      auto entry = [&](int row, int k) -> double & { return f[(int64_t)row * (BW + 1) * kTile + entry_at(BW + 1, k, km)]; };
-      if (q >= BW) entry(q - BW, 0) = lu.Lk[0];
-      else f[TileFac<BW>::fx(n) + (BW * BW + q) * kTile + km] = lu.Lk[0];
+  const Tabs<BW> tb = tabs_at<BW>(a.tabs, n);
+  const double k2 = mode_k((int)m, a.nxh, a.nz, a.lmfxr, a.lmfzr).k2;
+  double *f = (vop ? a.vf : a.fac[op]) + (m / kTile) * TileFac<BW>::size(n);
+  const int km = (int)(m % kTile);
+  double ca = 0.0, cb = 0.0;
+  if (!vop) {
+    cb = *a.dt_ptr * rkc(2, a.substep) * (op == 0 ? a.nu / a.pr : op == 1 ? a.nu : a.nu / a.pr2);
+    ca = 1.0 + cb * k2;
+  }
+  LuSweep<BW, 0, 0, true, TileU<BW>> lu;
+  lu.init(n, TileU<BW>{f + TileFac<BW>::bwd(n), f + TileFac<BW>::bx(n) + km, n, km});
+  const double2 bc[1] = {z2(0.0, 0.0)};
+  const double br[1] = {0.0};
+  double2 zc[1];
+  double zr[1];
+  for (int r = 1; r <= n; ++r) {
+    lu.step(r, [&](int rr, double *row, bool c) {
+      if (vop) vrow<BW>(tb, rr, n, k2, row, c);
+      else helm_row<BW>(tb, rr, n, ca, cb, row, c);
+    }, bc, br, zc, zr);
+    const int q = r - 1;  // 0-based
+    auto entry = [&](int row, int k) -> double & { return f[(int64_t)row * (BW + 1) * kTile + entry_at(BW + 1, k, km)]; };
+    if (q >= BW) entry(q - BW, 0) = lu.Lk[0];
+    else f[TileFac<BW>::fx(n) + (BW * BW + q) * kTile + km] = lu.Lk[0];
 #pragma unroll
-      for (int d = 1; d <= BW; ++d)
-        if (q >= d) entry(q - d, d) = lu.Lk[d] * lu.Lk[0];
-      if (q >= n - BW) {
-        double *x = f + TileFac<BW>::fx(n) + (q - (n - BW)) * BW * kTile + km;
+    for (int d = 1; d <= BW; ++d)
+      if (q >= d) entry(q - d, d) = lu.Lk[d] * lu.Lk[0];
+    if (q >= n - BW) {
+      double *x = f + TileFac<BW>::fx(n) + (q - (n - BW)) * BW * kTile + km;
 #pragma unroll
-        for (int d = BW + 1; d <= 2 * BW; ++d) x[(d - BW - 1) * kTile] = lu.Lk[d] * lu.Lk[0];
-      }
+      for (int d = BW + 1; d <= 2 * BW; ++d) x[(d - BW - 1) * kTile] = lu.Lk[d] * lu.Lk[0];
     }
   }
-  if (vop || !a.fcdt) return;
-  __syncwarp();
-  // every block has read the old mark by the time it counts
-  if (threadIdx.x == 0 && atomicAdd(a.fcount, 1u) + 1 == gridDim.x * gridDim.y) {
+  // thread 0 of every block has a mode; every block has read the old mark by the time it counts
+  if (!vop && a.fcdt && threadIdx.x == 0 && atomicAdd(a.fcount, 1u) + 1 == gridDim.x * gridDim.y) {
     *a.fcount = 0;
     *a.fcdt = *a.dt_ptr;
   }

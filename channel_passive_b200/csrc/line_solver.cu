@@ -41,7 +41,7 @@ struct HelmArgs {
 // ------------------------------------------------------------------------------------------
 // k_line_factor: one thread per mode and operator; op = blockIdx.y (0 theta, 1 g and phi, 2 theta2), or
 // v's operator with a.fac[0] null.  LuSweep's profile Crout LU, stored by tile.  A no-op while the
-// sets hold this dt (a fixed time step: 3 us against 112 us on 128x97x128 once a substep and run).
+// sets hold this dt (a fixed time step: 3 us against 117 us on 128x97x128 once a substep and run).
 // The sets and the dt they hold are written here together, by the last block to finish: it runs beside the
 // transforms, and whatever becomes of the substep after it, the mark is that of the sets.  (For the same
 // reason it does not look at the error flag: some blocks would leave and others not.)
@@ -100,8 +100,10 @@ constexpr int helm_planes(int nsc) { return 8 + 2 * (nsc - 1); }
 // The chain threads, in whole warps: 7 chains of kTile modes, 9 with a second scalar.
 constexpr int helm_chain_threads(int nsc) { return ((5 + 2 * nsc) * kTile + 31) / 32 * 32; }
 // Two blocks of eight warps an SM (128 registers a thread), 16 modes in flight.  Tiles of 4 modes in 3 or 4
-// blocks an SM were slower (64x65x64: 57 against 41 us, its 512 tiles take two waves), and so was every
-// shape whose registers spilled in the mat-vecs: local memory finds no L1 beside the lines.
+// blocks an SM were slower (64x65x64: 57 against 41 us, its 512 tiles take two waves), and so were shapes that
+// spilled more than these registers do (128 to 208 bytes at BW = 4): local memory finds no L1 beside the lines.
+// Above ny = 139 at BW = 4 (79 with two scalars) one block is resident.  64x65x64 FP64: 38 us with k_line_factor's
+// no-op, against 147 + 12 with k_helmholtz and k_assemble; 128x97x128 162 against 238 + 29.
 constexpr int kHelmThreads = 256;
 constexpr int kHelmBlocks = 2;  // resident blocks asked for
 
@@ -538,7 +540,8 @@ __global__ void __launch_bounds__(kHelmThreads, kHelmBlocks) k_lines(HelmArgs a)
 //   h_g = kx kz (f1 - f3) + (kz^2 - kx^2) f5 + D1 c(i kx f4 - i kz f2)
 //   h_theta = -(i kx f7 + i kz f9 + D1 c(f8)), with c(f) = D0^{-1} f.
 // At substep 1 also D2 D0^{-1} of the RK stores, and the control probes v(+-y_d) = w . v of the
-// substep's starting v.  k_hvhg (wavespace_split.cu) takes 77 us on 64x65x64 FP64, 37 us even on 16x33x16.
+// substep's starting v.  64x65x64 FP64: 38 us against 78 with k_hvhg (wavespace_split.cu), 16x33x16 23 against
+// 38, 128x97x128 150 against 132, where k_lines makes up for it.
 struct HvhgArgs {
   int n, nxh, nz, substep, nmodes;
   const void *P[11];

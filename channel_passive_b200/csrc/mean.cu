@@ -13,7 +13,7 @@ namespace {
 // (line 2: nu/pr, forced to the bulk value), a second scalar (line 3).  One block; warp l holds line l
 // in shared memory, its serial chains (real and imaginary parts, flux and store) a lane each and the
 // rest over all lanes, while warp 4 + l factors the line's operator.  One thread a line, with its work
-// lines in global memory, took 460 us at ny = 129, longer than the solver kernels beside it.
+// lines in global memory, took 464 us at ny = 129, longer than the solver kernels beside it; this takes 134.
 struct MeanArgs {
   int ny, substep, nsc;
   int64_t nmodes, ns;
